@@ -39,7 +39,7 @@ enum KernelId {
     K_IR, K_PCG_INIT_AMG32, K_PCG_ITER1_32, K_PCG_ITER2_AMG32, K_AMG_VCYCLE32, K_PERMUTE, K_GUESS, K_GNN,
     K_SNAPSHOT, K_BIR, K_ROUND_ELL, K_BICG3_INIT32, K_BICG3_1_32, K_BICG3_2_32, K_BICG3_3_32, K_BICG1_INIT32,
     K_BICG1_1_32, K_BICG1_2_32, K_BICG1_3_32, K_GRAD6, K_SCALAR, K_SCALAR_CLIP, K_EXCHANGE, K_LINE3, K_LINE1,
-    K_GNN_LAYERS, K_COUNT
+    K_GNN_LAYERS, K_SWEEP3, K_SWEEP1, K_COUNT
 };
 
 const char *kKernelNames[K_COUNT] = {
@@ -53,7 +53,7 @@ const char *kKernelNames[K_COUNT] = {
     "snapshot_pack", "bicg_refine_fp64_residual", "round_fp32", "bicg3_32_init", "bicg3_32_1_spmv",
     "bicg3_32_2_spmv", "bicg3_32_3_update", "bicg1_32_init", "bicg1_32_1_spmv", "bicg1_32_2_spmv",
     "bicg1_32_3_update", "lsq_gradients_scalars", "scalar_assemble", "scalar_clip_negative", "particle_exchange",
-    "line_sweep3_32", "line_sweep1_32", "gnn_layers"};
+    "line_sweep3_32", "line_sweep1_32", "gnn_layers", "line_sweep3_64", "line_sweep1_64"};
 
 constexpr int PCG_BATCH = 16;   // iterations per status read (even: ping-pong buffers)
 constexpr int PCG_AMG_BATCH = 4;
@@ -175,6 +175,10 @@ struct mc_flow {
     int line_ex = 0;
     LineSystem line3{}, line1{};
     float *line_scratch = nullptr;
+    // the same lines for the FP64 sweeps (momentum, temperature, scalars)
+    LineRows64 line64{};              // diag and off are set for each solve
+    SweepState<3> *sweep3 = nullptr, *h_sweep3 = nullptr;  // device; pinned
+    SweepState<1> *sweep1 = nullptr, *h_sweep1 = nullptr;
     // initial guess of the pressure correction
     double *pp_prev = nullptr;        // previous converged correction [N]
     GuessState *gs = nullptr;
@@ -774,6 +778,64 @@ int solve_bicg(mc_flow *h, const Ell &A, const BicgVectors<R> &v, BicgState<R> *
     return worst;
 }
 
+// Sweeps of a line-sweep solve launched together (the momentum and transport
+// solves of the benchmark flow take four at 1e-8, five or six at 1e-13; a
+// sweep launched after the solve is done costs about a microsecond, reading
+// the state and launching again about fifteen).
+constexpr int SWEEP_BATCH = 6;
+constexpr int SWEEP_MAX = 40;
+// BiCGStab is kept where max_iters is below this: its iterations are what the
+// caller then bounds.
+constexpr int SWEEP_MIN_ITERS = 50;
+
+// The solve by FP64 x-line sweeps (krylov.cuh), x[j] the solutions and
+// `scratch` [R][N] the other iterate.  Returns MC_OK with *used set when every
+// system met ||b - A x|| <= u_rtol ||b||; *used = false when the splitting is
+// not the faster method here -- a sweep that does not halve the residual of an
+// open system (a BiCGStab iteration moves four times a sweep's bytes and takes
+// about a decade off), or a non-finite value -- and the caller runs BiCGStab
+// from zero.
+template <int R>
+int solve_sweeps(mc_flow *h, const double *diag, const double *off, const double *b, double *const (&x)[R],
+                 double *scratch, SweepState<R> *st, SweepState<R> *hs, int iters_out[R], bool *used)
+{
+    *used = false;
+    if (h->line_ex == 0 || h->prm.max_iters < SWEEP_MIN_ITERS) return MC_OK;
+    LineRows64 L = h->line64;
+    L.diag = diag;
+    L.off = off;
+    SweepVectors<R> v{};
+    for (int j = 0; j < R; j++) {
+        v.x[0][j] = x[j];
+        v.x[1][j] = scratch + (size_t)j * h->N;
+    }
+    v.b = b;
+    v.partials = h->partials;
+    v.counter = h->counter;
+    v.st = st;
+    for (int k = 0; k < SWEEP_MAX;) {
+        for (int q = 0; q < SWEEP_BATCH; q++, k++)
+            launch(h, R == 3 ? K_SWEEP3 : K_SWEEP1, [&] { line_sweep64<R>(h->stream, L, v, k, h->prm.u_rtol); });
+        const int rc = check_launch(h);
+        if (rc) return rc;
+        CUDA_TRY(h, cudaMemcpyAsync(hs, st, sizeof(SweepState<R>), cudaMemcpyDeviceToHost, h->stream));
+        CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+        flush_timing(h);
+        if (hs->nonfinite) return MC_OK;
+        if (hs->all_done) break;
+        for (int j = 0; j < R; j++)
+            if (!hs->done[j] && !(hs->rr[j] <= 0.25 * hs->rr_prev[j])) return MC_OK;
+    }
+    if (!hs->all_done) return MC_OK;
+    if (hs->where == 1)
+        for (int j = 0; j < R; j++)
+            CUDA_TRY(h, cudaMemcpyAsync(v.x[0][j], v.x[1][j], (size_t)h->N * sizeof(double), cudaMemcpyDeviceToDevice,
+                                        h->stream));
+    for (int j = 0; j < R; j++) iters_out[j] = hs->iter[j];
+    *used = true;
+    return MC_OK;
+}
+
 // FP64 iterative refinement around FP32 BiCGStab solves (momentum, R = 3;
 // temperature, R = 1): each inner solve works on the row-scaled system
 // D^-1 A e = D^-1 r (FP32 copies from round_ell, D = diag A) and asks for
@@ -1096,7 +1158,10 @@ int stage_momentum(mc_flow *h, mc_iter_stats *st)
         rc = solve_bicg_refined<3>(h, momentum_matrix(h), A32, h->bi3, h->bo3, h->h_bi3, h->h_bo3, &h->g_b3_32,
                                    &h->l_b3_32, K_BICG3_INIT32, K_BICG3_1_32, its);
     } else {
-        rc = solve_bicg<3>(h, momentum_matrix(h), h->b3, h->h_b3, &h->g_b3, &h->l_b3, K_BICG3_INIT, K_BICG3_1, its);
+        bool swept = false;
+        rc = solve_sweeps<3>(h, h->AU, h->off_m, h->b_m, h->b3.x, h->b3.s, h->sweep3, h->h_sweep3, its, &swept);
+        if (!rc && !swept)
+            rc = solve_bicg<3>(h, momentum_matrix(h), h->b3, h->h_b3, &h->g_b3, &h->l_b3, K_BICG3_INIT, K_BICG3_1, its);
     }
     if (st)
         for (int j = 0; j < 3; j++) st->momentum_iters[j] = its[j];
@@ -1259,7 +1324,11 @@ int stage_temperature(mc_flow *h, mc_iter_stats *st)
         rc = solve_bicg_refined<1>(h, temperature_matrix(h), A32, h->bi1, h->bo1, h->h_bi1, h->h_bo1, &h->g_b1_32,
                                    &h->l_b1_32, K_BICG1_INIT32, K_BICG1_1_32, its);
     } else {
-        rc = solve_bicg<1>(h, temperature_matrix(h), h->b1, h->h_b1, &h->g_b1, &h->l_b1, K_BICG1_INIT, K_BICG1_1, its);
+        bool swept = false;
+        rc = solve_sweeps<1>(h, h->diag_t, h->off_t, h->b_t, h->b1.x, h->b1.s, h->sweep1, h->h_sweep1, its, &swept);
+        if (!rc && !swept)
+            rc = solve_bicg<1>(h, temperature_matrix(h), h->b1, h->h_b1, &h->g_b1, &h->l_b1, K_BICG1_INIT, K_BICG1_1,
+                               its);
     }
     if (st) st->temperature_iters = its[0];
     return rc;
@@ -1310,8 +1379,12 @@ int stage_scalar(mc_flow *h, int field, mc_iter_stats *st)
     int rc = check_launch(h);
     if (rc) return rc;
     int its[1] = {0};
-    const int solve_rc =
-        solve_bicg<1>(h, temperature_matrix(h), h->bs, h->h_b1, &h->g_bs, &h->l_bs, K_BICG1_INIT, K_BICG1_1, its);
+    bool swept = false;
+    int solve_rc =
+        solve_sweeps<1>(h, h->diag_t, h->off_t, h->b_t, h->bs.x, h->bs.s, h->sweep1, h->h_sweep1, its, &swept);
+    if (!solve_rc && !swept)
+        solve_rc =
+            solve_bicg<1>(h, temperature_matrix(h), h->bs, h->h_b1, &h->g_bs, &h->l_bs, K_BICG1_INIT, K_BICG1_1, its);
     if (solve_rc == MC_ERR_CUDA) return solve_rc;
     CUDA_TRY(h, cudaMemcpyAsync(phi, h->xs, (size_t)h->N * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
     if (type == SC_TERBTE || type == SC_TERBED) {
@@ -1384,6 +1457,8 @@ int allocate(mc_flow *h)
     for (int k = 0; k < 8; k++) add(&bic[k], 3 * N * 8);
     add(&h->b3.st, sizeof(BicgState<3>));
     add(&h->b1.st, sizeof(BicgState<1>));
+    add(&h->sweep3, sizeof(SweepState<3>));
+    add(&h->sweep1, sizeof(SweepState<1>));
     add(&h->pp_prev, N * 8);
     add(&h->dcode, N * 4);
     add(&h->gs, sizeof(GuessState));
@@ -1422,6 +1497,8 @@ int allocate(mc_flow *h)
     CUDA_TRY(h, cudaMallocHost((void **)&h->h_b3, sizeof(BicgState<3>)));
     CUDA_TRY(h, cudaMallocHost((void **)&h->h_b1, sizeof(BicgState<1>)));
     CUDA_TRY(h, cudaMallocHost((void **)&h->h_scalars, 8 * sizeof(double)));
+    CUDA_TRY(h, cudaMallocHost((void **)&h->h_sweep3, sizeof(SweepState<3>)));
+    CUDA_TRY(h, cudaMallocHost((void **)&h->h_sweep1, sizeof(SweepState<1>)));
     return MC_OK;
 }
 
@@ -2128,6 +2205,25 @@ int mc_flow_create(const mc_mesh_view *mesh, const mc_flow_params *params, mc_fl
                         for (int d = 0; d < 6; d++) h->dc_rows.doff[(pos >> (3 * d)) & 7u] = doff[d];
                         h->hcode.swap(code);
                     }
+                    if (h->line_ex > 0) {
+                        // positions of the directions in the FP64 rows; in slot
+                        // order (no common order of the directions) the kernel
+                        // finds a direction's slot from the row's code word
+                        LineRows64 &L = h->line64;
+                        L.N = (int)N;
+                        L.ex = h->line_ex;
+                        L.code = h->rows.code ? nullptr : h->dcode;
+                        const int *off6 = h->rows.code ? h->dc_rows.doff : h->dc.doff;
+                        int q = 0;
+                        for (int d = 0; d < 6; d++) {
+                            if (off6[d] == -1) L.xm = d;
+                            else if (off6[d] == 1) L.xp = d;
+                            else {
+                                L.yz[q] = d;
+                                L.yzoff[q++] = off6[d];
+                            }
+                        }
+                    }
                 }
             }
             const int form = pressure_copy_form();
@@ -2216,7 +2312,8 @@ int mc_flow_destroy(mc_flow *h)
     if (h->xin_mem) cudaFree(h->xin_mem);
     for (cudaGraphExec_t g : {h->g_bs, h->l_bs})
         if (g) cudaGraphExecDestroy(g);
-    for (void *p : {(void *)h->h_bi3, (void *)h->h_bi1, (void *)h->h_bo3, (void *)h->h_bo1})
+    for (void *p : {(void *)h->h_bi3, (void *)h->h_bi1, (void *)h->h_bo3, (void *)h->h_bo1, (void *)h->h_sweep3,
+                    (void *)h->h_sweep1})
         if (p) cudaFreeHost(p);
     if (h->side) cudaStreamSynchronize(h->side);  // no inverse still being formed into freed memory
     if (h->stream) cudaStreamDestroy(h->stream);

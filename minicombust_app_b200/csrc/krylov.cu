@@ -32,7 +32,7 @@ __device__ __forceinline__ bool finite(double x) { return isfinite(x); }
 
 } // namespace
 
-int krylov_grid(int N)
+static int krylov_sms()
 {
     static int sms = 0;
     if (sms == 0) {
@@ -41,8 +41,13 @@ int krylov_grid(int N)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (sms <= 0) sms = 148;
     }
+    return sms;
+}
+
+int krylov_grid(int N)
+{
     const int need = (N + MCB_THREADS - 1) / MCB_THREADS;
-    return std::max(1, std::min(need, sms * MCB_KRYLOV_BLOCKS_PER_SM));
+    return std::max(1, std::min(need, krylov_sms() * MCB_KRYLOV_BLOCKS_PER_SM));
 }
 
 // ---------------------------------------------------------------------- PCG
@@ -1285,6 +1290,207 @@ template void line_step<1>(cudaStream_t, const LineSystem &, const float *, cons
                            const BirVectors<1> *);
 template void line_step<3>(cudaStream_t, const LineSystem &, const float *, const float *, float *, int,
                            const BirVectors<3> *);
+
+// ---------------------------------------------------- FP64 x-line sweeps
+//
+// HBM bound: a sweep streams the row once for all R systems, 56 bytes of
+// matrix and per system b, x_k and x_{k+1} (24 bytes; 16 for the first sweep,
+// which reads three of the seven matrix values).  A momentum solve to 1e-8
+// takes four sweeps, 448 bytes per row, where BiCGStab takes 8 to 10
+// iterations of 520: a plain FP64 timestep of the 2 x 128^3 box 48.6 -> 26.8 ms,
+// with errors against 64-bit solves ten times smaller.
+// One warp per line: the cells' affine maps e_i = p_i + q_i e_{i-1} are formed
+// from independent coalesced loads into shared memory, then composed by warp
+// scans of 32 cells and a carry.  The residual of the iterate read is the
+// right-hand side the map is formed from less its own diagonal and -x terms,
+// so convergence costs no extra pass over the matrix; the iterate returned is
+// one sweep better than the one tested.
+template <int R, bool DIR>
+__device__ __forceinline__ double line_value(const LineRows64 &L, size_t i, uint32_t cw, int d)
+{
+    if (DIR) return L.off[(size_t)d * L.N + i];
+    double v = 0.0;
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+        if (((cw >> (3 * k)) & 7u) == (unsigned)d) v = L.off[(size_t)k * L.N + i];
+    return v;
+}
+
+template <int R>
+struct SweepPtrs {
+    const double *in[R];
+    double *out[R];
+};
+
+// Resident blocks of 256 per SM: 3 x 64 KB of maps for three systems (24
+// warps hold about 160 KB of loads in flight per SM), 4 for one.
+template <int R>
+constexpr int sweep_blocks() { return R == 1 ? 4 : 3; }
+
+template <int R, bool DIR, bool FIRST>
+__global__ void __launch_bounds__(256, sweep_blocks<R>())
+    k_line_sweep64(LineRows64 L, SweepVectors<R> v, SweepPtrs<R> x, int to, double rtol)
+{
+    pdl_wait();
+    extern __shared__ double sweep_smem[];
+    __shared__ double sw[R][32];
+    SweepState<R> *st = v.st;
+    if (!FIRST && st->all_done) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int N = L.N, ex = L.ex, lines = N / ex;
+    double *sq = sweep_smem + (size_t)warp * ex * (R + 1);  // q[ex], then p[R][ex]
+    double *sp = sq + ex;
+    double acc[R];
+#pragma unroll
+    for (int j = 0; j < R; j++) acc[j] = 0.0;
+    for (int line = blockIdx.x * nw + warp; line < lines; line += gridDim.x * nw) {
+        const size_t base = (size_t)line * ex;
+#pragma unroll 1
+        for (int c = lane; c < ex; c += 32) {
+            const size_t i = base + c;
+            const uint32_t cw = DIR ? 0u : L.code[i];
+            const double d = L.diag[i];
+            const double a = line_value<R, DIR>(L, i, cw, L.xm);
+            double rhs[R];
+#pragma unroll
+            for (int j = 0; j < R; j++) rhs[j] = v.b[(size_t)j * N + i];
+            if (FIRST) {
+#pragma unroll
+                for (int j = 0; j < R; j++) acc[j] += rhs[j] * rhs[j];
+            } else {
+                const double op = line_value<R, DIR>(L, i, cw, L.xp);
+                double oy[4];
+                size_t nb[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    oy[u] = line_value<R, DIR>(L, i, cw, L.yz[u]);
+                    nb[u] = (size_t)min(max((long)i + L.yzoff[u], 0L), (long)N - 1);
+                }
+                const size_t im = c > 0 ? i - 1 : i, ip = c + 1 < ex ? i + 1 : i;
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    const double *__restrict__ xin = x.in[j];
+                    const double x0 = xin[i], xm = xin[im], xp = xin[ip];
+                    double xy[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) xy[u] = xin[nb[u]];
+                    double s = rhs[j];
+                    if (c + 1 < ex) s -= op * xp;
+#pragma unroll
+                    for (int u = 0; u < 4; u++) s -= oy[u] * xy[u];
+                    rhs[j] = s;
+                    double res = s - d * x0;
+                    if (c > 0) res -= a * xm;
+                    acc[j] += res * res;
+                }
+            }
+            const double rb = 1.0 / d;
+            sq[c] = -a * rb;
+#pragma unroll
+            for (int j = 0; j < R; j++) sp[j * ex + c] = rhs[j] * rb;
+        }
+        __syncwarp();
+        double carry[R];
+#pragma unroll
+        for (int j = 0; j < R; j++) carry[j] = 0.0;
+        for (int c0 = 0; c0 < ex; c0 += 32) {
+            const int c = c0 + lane;
+            double p[R], q = 1.0;
+#pragma unroll
+            for (int j = 0; j < R; j++) p[j] = 0.0;
+            if (c < ex) {
+                q = sq[c];
+#pragma unroll
+                for (int j = 0; j < R; j++) p[j] = sp[j * ex + c];
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                double pu[R];
+#pragma unroll
+                for (int j = 0; j < R; j++) pu[j] = __shfl_up_sync(0xffffffffu, p[j], o);
+                const double qu = __shfl_up_sync(0xffffffffu, q, o);
+                if (lane >= o) {
+#pragma unroll
+                    for (int j = 0; j < R; j++) p[j] += q * pu[j];
+                    q *= qu;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < R; j++) {
+                const double e = p[j] + q * carry[j];
+                if (c < ex) x.out[j][base + c] = e;
+                carry[j] = __shfl_sync(0xffffffffu, e, 31);
+            }
+        }
+        __syncwarp();  // the maps are read before the next line's replace them
+    }
+    if (publish_sums<R>(acc, v.partials, v.counter, sw)) {
+        double tot[R];
+        reduce_sums<R>(tot, v.partials, v.counter, sw);
+        if (threadIdx.x == 0) {
+            int all = 1, bad = 0;
+            const int sweeps = FIRST ? 1 : st->sweeps + 1;
+            for (int j = 0; j < R; j++) {
+                bad |= !finite(tot[j]);
+                if (FIRST) {
+                    st->bb[j] = st->rr[j] = st->rr_prev[j] = tot[j];
+                    st->tol2[j] = rtol * rtol * tot[j];
+                    st->done[j] = tot[j] == 0.0;
+                    st->iter[j] = 1;
+                } else if (!st->done[j]) {
+                    st->rr_prev[j] = st->rr[j];
+                    st->rr[j] = tot[j];
+                    st->iter[j] = sweeps;
+                    st->done[j] = tot[j] <= st->tol2[j];
+                }
+                all &= st->done[j];
+            }
+            st->nonfinite = bad;
+            st->sweeps = sweeps;
+            st->where = to;
+            st->all_done = all | bad;
+        }
+    }
+}
+
+namespace {
+// Dynamic shared memory the sweeps may take: three blocks of it fit an SM.
+constexpr size_t SWEEP_SMEM_MAX = 72 * 1024;
+
+template <int R, bool DIR, bool FIRST>
+void launch_line_sweep64(cudaStream_t s, const LineRows64 &L, const SweepVectors<R> &v, int from, double rtol)
+{
+    const size_t per_warp = (size_t)L.ex * (R + 1) * sizeof(double);
+    int warps = 8;
+    while (warps > 1 && warps * per_warp > SWEEP_SMEM_MAX) warps >>= 1;
+    auto k = k_line_sweep64<R, DIR, FIRST>;
+    // (a per-device attribute of the function; setting it again costs nothing)
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SWEEP_SMEM_MAX);
+    const int lines = L.N / L.ex;
+    const int grid = std::min({(lines + warps - 1) / warps, line_sweep64_blocks(L.N), krylov_sms() * sweep_blocks<R>()});
+    SweepPtrs<R> x{};
+    for (int j = 0; j < R; j++) {
+        x.in[j] = v.x[from][j];
+        x.out[j] = v.x[from ^ 1][j];
+    }
+    pdl_launch(k, dim3(grid), dim3(32 * warps), warps * per_warp, s, L, v, x, from ^ 1, rtol);
+}
+} // namespace
+
+int line_sweep64_blocks(int N) { return krylov_grid(N); }
+
+template <int R>
+void line_sweep64(cudaStream_t s, const LineRows64 &L, const SweepVectors<R> &v, int k, double rtol)
+{
+    if (L.code)
+        k == 0 ? launch_line_sweep64<R, false, true>(s, L, v, 0, rtol)
+               : launch_line_sweep64<R, false, false>(s, L, v, k & 1, rtol);
+    else
+        k == 0 ? launch_line_sweep64<R, true, true>(s, L, v, 0, rtol)
+               : launch_line_sweep64<R, true, false>(s, L, v, k & 1, rtol);
+}
+template void line_sweep64<1>(cudaStream_t, const LineRows64 &, const SweepVectors<1> &, int, double);
+template void line_sweep64<3>(cudaStream_t, const LineRows64 &, const SweepVectors<3> &, int, double);
 
 void round_ell(cudaStream_t s, int N, const double *diag, const double *off, const uint32_t *code, float *diag32,
                float *off32)

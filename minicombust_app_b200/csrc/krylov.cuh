@@ -293,6 +293,43 @@ template <int R>
 void line_step(cudaStream_t s, const LineSystem &L, const float *r, const float *e_prev, float *e_new, int first,
                const BirVectors<R> *add = nullptr);
 
+// FP64 x-line sweeps: the whole momentum or transport solve as the splitting
+// iteration x_{k+1} = M^-1 (b - (A - M) x_k), M the diagonal and the -x
+// couplings of each x-line, from x_0 = 0, on a structured box whose cells run
+// x-fastest along whole lines.  Each sweep also forms the true residual of
+// the iterate it reads.
+struct LineRows64 {
+    int N = 0;
+    int ex = 0;                 // cells per x-line (<= 1024)
+    int xm = 0, xp = 0;         // rows of off holding the -x and +x couplings
+    int yz[4] = {0, 0, 0, 0};   // the other four
+    int yzoff[4] = {0, 0, 0, 0};
+    const uint32_t *code = nullptr;  // null: off rows are positions; else slot order with these direction codes
+                                     // (xm, xp and yz are then directions)
+    const double *diag = nullptr;
+    const double *off = nullptr;     // [6][N]
+};
+template <int R>
+struct SweepState {
+    double bb[R], rr[R], rr_prev[R], tol2[R];
+    int iter[R], done[R];
+    int all_done, nonfinite, sweeps, where;  // where: buffer (0 or 1) the last sweep wrote
+};
+// Sweep number k (0: from zero, which also sets the tolerance rtol ||b||):
+// reads x[k & 1], writes x[(k & 1) ^ 1]; sweeps after the solve is done do
+// nothing.  grid blocks of the launch: line_sweep64_grid.
+template <int R>
+struct SweepVectors {
+    double *x[2][R];            // the two iterates
+    const double *b;            // [R][N]
+    double *partials;           // R doubles for each block
+    unsigned int *counter;
+    SweepState<R> *st;
+};
+template <int R>
+void line_sweep64(cudaStream_t s, const LineRows64 &L, const SweepVectors<R> &v, int k, double rtol);
+int line_sweep64_blocks(int N);  // upper bound on the blocks of a launch over N rows
+
 enum { KRYLOV_OK = 0, KRYLOV_NOT_CONVERGED = 1, KRYLOV_NONFINITE = 2 };
 
 // Grid size used by the Krylov kernels for N rows.

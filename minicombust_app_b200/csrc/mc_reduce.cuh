@@ -99,4 +99,66 @@ __device__ inline void reduce_partials(double (&out)[K], const double *partials,
     if (threadIdx.x == 0) *counter = 0u;
 }
 
+__device__ __forceinline__ double warp_sum_all(double v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Block sums of K values by warp shuffles (any block size that is a multiple
+// of 32): two barriers whatever K is.  sw: [K][32] shared; result in every
+// lane of warp 0.
+template <int K>
+__device__ __forceinline__ void block_sums(double (&v)[K], double (*sw)[32])
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    __syncthreads();  // sw may still be read from a previous reduction
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        v[k] = warp_sum_all(v[k]);
+        if (lane == 0) sw[k][warp] = v[k];
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] = warp_sum_all(lane < nw ? sw[k][lane] : 0.0);
+    }
+}
+
+// publish_partials / reduce_partials with shuffle sums.
+template <int K>
+__device__ __forceinline__ bool publish_sums(const double (&v)[K], double *partials, unsigned int *counter,
+                                             double (*sw)[32])
+{
+    __shared__ bool am_last;
+    double b[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) b[k] = v[k];
+    block_sums<K>(b, sw);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < K; k++) partials[(size_t)blockIdx.x * K + k] = b[k];
+        __threadfence();
+        am_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    return am_last;
+}
+
+// In the last block: the partials of all blocks in a fixed order (thread t
+// takes blocks t, t + blockDim, ...).  Result in thread 0.
+template <int K>
+__device__ __forceinline__ void reduce_sums(double (&out)[K], const double *partials, unsigned int *counter,
+                                            double (*sw)[32])
+{
+#pragma unroll
+    for (int k = 0; k < K; k++) out[k] = 0.0;
+    for (unsigned int b = threadIdx.x; b < gridDim.x; b += blockDim.x)
+#pragma unroll
+        for (int k = 0; k < K; k++) out[k] += __ldcg(partials + (size_t)b * K + k);
+    block_sums<K>(out, sw);
+    if (threadIdx.x == 0) *counter = 0u;
+}
+
 } // namespace mcb

@@ -1,0 +1,59 @@
+"""The FP64 x-line sweeps (momentum, temperature and scalar solves on boxes
+whose cells run x-fastest) against the CPU oracle, whose solves are BiCGStab:
+line lengths at the edges of the 32-cell scan chunks and of the shared-memory
+split, meshes of a few lines, and a flow across the lines with a long time
+step, where the splitting converges too slowly and BiCGStab takes over.
+
+Solves run to 1e-12 on both sides; fields agree to 1e-9 of their maximum, the
+parity gate of the other whole-pass tests (the transient term bounds the
+matrices' condition, so 1e-12 residuals leave errors far below it).
+"""
+import numpy as np
+import pytest
+
+from checkers import SIMPLE, Oracle, noisy_initial_fields, oracle_mesh, oracle_params
+from minicombust_app_b200 import flow
+
+pytestmark = pytest.mark.gpu
+
+BASE = {"U": 50.0, "V": 0.0, "W": 0.0, "P": 4000.0, "TEM": 1500.0}
+
+
+def run_both(dims, passes=2, base=BASE, **kw):
+    lengths = (0.2, 0.1, 0.1)
+    p = flow.default_params(flow.MODE_SIMPLE, u_rtol=1e-12, p_rtol=1e-12, **kw)
+    solver = flow.FlowSolver(flow.Mesh.box(*dims, *lengths), params=p)
+    okw = {"u_rtol": 1e-12, "p_rtol": 1e-12}
+    if "delta" in kw:
+        okw["delta"] = kw["delta"]
+    orc = Oracle(oracle_mesh(*dims, *lengths), oracle_params(SIMPLE, scalars=p.transport_scalars, **okw))
+    for name, vals in noisy_initial_fields(solver.N, base, 1).items():
+        for s in (solver, orc):
+            a = s.field(name)
+            a[:solver.N] = vals
+            s.set_field(name, a)
+    for _ in range(passes):
+        solver.simple_iteration()
+        orc.step()
+    for name in BASE:
+        a, b = solver.field(name), orc.field(name)
+        assert np.abs(a - b).max() <= 1e-9 * np.abs(b).max(), (dims, name)
+    st = solver.last_stats
+    solver.close()
+    return st
+
+
+@pytest.mark.parametrize("dims", [(2, 3, 3), (31, 3, 2), (32, 2, 5), (33, 5, 3), (257, 2, 2), (513, 2, 2),
+                                  (1024, 2, 2)])
+def test_sweeps_match_oracle(gpu, dims):
+    st = run_both(dims)
+    # a sweep gains about three decades on this flow: 1e-12 within one batch
+    assert 1 <= max(st.momentum_iters) <= 12 and 1 <= st.temperature_iters <= 12
+
+
+def test_scalars_by_sweeps_match_oracle(gpu):
+    run_both((33, 6, 5), transport_scalars=1)
+
+
+def test_cross_flow_falls_back_to_bicgstab(gpu):
+    run_both((12, 24, 6), passes=1, base={**BASE, "U": 1.0, "V": 80.0}, delta=1e-2)
