@@ -22,6 +22,7 @@
 #include "flow_kernels.cuh"
 #include "gnn.cuh"
 #include "krylov.cuh"
+#include "krylov_team.cuh"
 #include "mc_internal.h"
 #include "mc_reduce.cuh"
 #include "mesh_setup.h"
@@ -39,7 +40,7 @@ enum KernelId {
     K_IR, K_PCG_INIT_AMG32, K_PCG_ITER1_32, K_PCG_ITER2_AMG32, K_AMG_VCYCLE32, K_PERMUTE, K_GUESS, K_GNN,
     K_SNAPSHOT, K_BIR, K_ROUND_ELL, K_BICG3_INIT32, K_BICG3_1_32, K_BICG3_2_32, K_BICG3_3_32, K_BICG1_INIT32,
     K_BICG1_1_32, K_BICG1_2_32, K_BICG1_3_32, K_GRAD6, K_SCALAR, K_SCALAR_CLIP, K_EXCHANGE, K_LINE3, K_LINE1,
-    K_GNN_LAYERS, K_SWEEP3, K_SWEEP1, K_COUNT
+    K_GNN_LAYERS, K_SWEEP3, K_SWEEP1, K_PCG_TEAM, K_BICG1_TEAM, K_COUNT
 };
 
 const char *kKernelNames[K_COUNT] = {
@@ -53,7 +54,8 @@ const char *kKernelNames[K_COUNT] = {
     "snapshot_pack", "bicg_refine_fp64_residual", "round_fp32", "bicg3_32_init", "bicg3_32_1_spmv",
     "bicg3_32_2_spmv", "bicg3_32_3_update", "bicg1_32_init", "bicg1_32_1_spmv", "bicg1_32_2_spmv",
     "bicg1_32_3_update", "lsq_gradients_scalars", "scalar_assemble", "scalar_clip_negative", "particle_exchange",
-    "line_sweep3_32", "line_sweep1_32", "gnn_layers", "line_sweep3_64", "line_sweep1_64"};
+    "line_sweep3_32", "line_sweep1_32", "gnn_layers", "line_sweep3_64", "line_sweep1_64",
+    "pcg_team", "bicg1_team"};
 
 constexpr int PCG_BATCH = 16;   // iterations per status read (even: ping-pong buffers)
 constexpr int PCG_AMG_BATCH = 4;
@@ -356,7 +358,10 @@ Ell temperature_matrix(mc_flow *h) { return Ell{h->N, h->diag_t, h->off_t, h->co
 
 int krylov_status_to_mc(int s)
 {
-    return s == KRYLOV_OK ? MC_OK : (s == KRYLOV_NONFINITE ? MC_ERR_NONFINITE : MC_ERR_NOT_CONVERGED);
+    return s == KRYLOV_OK          ? MC_OK
+           : s == KRYLOV_NONFINITE ? MC_ERR_NONFINITE
+           : s == KRYLOV_TIMEOUT   ? MC_ERR_TIMEOUT
+                                   : MC_ERR_NOT_CONVERGED;
 }
 
 // Graph of one batch of iterations, captured on first use.
@@ -554,6 +559,10 @@ int after_pressure_solve(mc_flow *h)
 
 int launch_deferred_inverse(mc_flow *h);
 
+// Barrier memory of the team solvers: a word of the counters' block and the
+// block partials (a team runs alone on the handle's stream).
+TeamMem team_mem(mc_flow *h) { return TeamMem{h->counter + 16, h->partials}; }
+
 int solve_pressure(mc_flow *h, double abs_floor, int *iters, double *relres, double *bnorm)
 {
     const Ell A = pressure_matrix(h);
@@ -563,6 +572,24 @@ int solve_pressure(mc_flow *h, double abs_floor, int *iters, double *relres, dou
     const int use_x0 = select_guess(h, A, v.b, v.st, v.x);
     h->guess_used = use_x0 != 0;
     if (const int rl = launch_deferred_inverse(h)) return rl;
+    if (!amg) {
+        // small systems: the whole solve in one kernel
+        bool team = false;
+        launch(h, K_PCG_TEAM, [&] {
+            team = pcg_team(h->stream, A, v, h->prm.p_rtol, abs_floor, h->prm.max_iters, use_x0, team_mem(h));
+        });
+        if (team) {
+            CUDA_TRY(h, cudaMemcpyAsync(h->h_pcg, v.st, sizeof(PcgState), cudaMemcpyDeviceToHost, h->stream));
+            CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+            flush_timing(h);
+            const PcgState &s = *h->h_pcg;
+            *iters = s.iter;
+            *bnorm = std::sqrt(s.bb);
+            *relres = s.bb > 0 ? std::sqrt(s.rr / s.bb) : 0.0;
+            return krylov_status_to_mc(s.status);
+        }
+        h->launches--;
+    }
     if (amg) {
         launch(h, K_PCG_INIT_AMG,
                [&] { pcg_init_amg(h->stream, A, v, h->prm.p_rtol, abs_floor, h->prm.max_iters, 1, use_x0); });
@@ -745,6 +772,21 @@ template <int R>
 int solve_bicg(mc_flow *h, const Ell &A, const BicgVectors<R> &v, BicgState<R> *hs, cudaGraphExec_t *exec,
                cudaGraphExec_t *loop, int kid_init, int kid1, int iters_out[R])
 {
+    if constexpr (R == 1) {  // small systems: the whole solve in one kernel
+        bool team = false;
+        launch(h, K_BICG1_TEAM, [&] {
+            team = bicg_team(h->stream, A, v.b, v.x[0], h->pv.zp[0], v.v[0], v.v[1], v.st, h->prm.u_rtol,
+                             h->prm.max_iters, team_mem(h));
+        });
+        if (team) {
+            CUDA_TRY(h, cudaMemcpyAsync(hs, v.st, sizeof(BicgState<R>), cudaMemcpyDeviceToHost, h->stream));
+            CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+            flush_timing(h);
+            iters_out[0] = hs->iter[0];
+            return krylov_status_to_mc(hs->status[0]);
+        }
+        h->launches--;
+    }
     launch(h, kid_init, [&] { bicg_init<R>(h->stream, A, v, h->prm.u_rtol, h->prm.max_iters); });
     int rc = check_launch(h);
     if (rc) return rc;

@@ -330,7 +330,7 @@ template <int R>
 void line_sweep64(cudaStream_t s, const LineRows64 &L, const SweepVectors<R> &v, int k, double rtol);
 int line_sweep64_blocks(int N);  // upper bound on the blocks of a launch over N rows
 
-enum { KRYLOV_OK = 0, KRYLOV_NOT_CONVERGED = 1, KRYLOV_NONFINITE = 2 };
+enum { KRYLOV_OK = 0, KRYLOV_NOT_CONVERGED = 1, KRYLOV_NONFINITE = 2, KRYLOV_TIMEOUT = 3 };
 
 // Grid size used by the Krylov kernels for N rows.
 int krylov_grid(int N);

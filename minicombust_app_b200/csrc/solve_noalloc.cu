@@ -25,6 +25,7 @@
 #include <mutex>
 
 #include "krylov.cuh"
+#include "krylov_team.cuh"
 #include "mc_reduce.cuh"
 #include "minicombust_flow.h"
 
@@ -41,11 +42,12 @@ constexpr int kMaxBlocks = (kMaxRows + MCB_THREADS - 1) / MCB_THREADS;
 constexpr int kPartialsPerBlock = 8;
 static_assert(MCB_THREADS == 256, "scratch partitioning assumes 256-thread Krylov blocks");
 static_assert(kPartialsPerBlock >= 2, "BiCGStab with one right-hand side publishes 2 partials per block");
-constexpr size_t kStatusDoubles = 64;             // counter (first 8 bytes) + BicgState<1>
+constexpr size_t kStatusDoubles = 64;             // counter (first 8 bytes) + BicgState<1> + the team's barrier word
+constexpr size_t kArriveDouble = 48;              // where that word is
 constexpr size_t kScratchDoubles =
     (size_t)kVectors * kMaxRows + (size_t)kMaxBlocks * kPartialsPerBlock + kStatusDoubles;
 
-static_assert(sizeof(mcb::BicgState<1>) + 8 <= kStatusDoubles * sizeof(double), "status block too small");
+static_assert(sizeof(mcb::BicgState<1>) + 8 <= kArriveDouble * sizeof(double), "status block too small");
 
 static __device__ __align__(256) double g_scratch[kScratchDoubles];
 
@@ -103,11 +105,24 @@ extern "C" int mc_solve_bicgstab_noalloc(int n, const double *diag, const double
     // it was interrupted, so clear it (and the status) every time.
     if (cudaMemsetAsync(status, 0, kStatusDoubles * sizeof(double), s) != cudaSuccess) return MC_ERR_CUDA;
     const mcb::Ell A{n, diag, off, col};
+    mcb::BicgState<1> hs{};
+    auto status_of = [&]() -> int {
+        if (iterations) *iterations = hs.iter[0];
+        if (hs.status[0] == mcb::KRYLOV_NONFINITE) return MC_ERR_NONFINITE;
+        if (hs.status[0] == mcb::KRYLOV_TIMEOUT) return MC_ERR_TIMEOUT;
+        return hs.status[0] == mcb::KRYLOV_OK ? MC_OK : MC_ERR_NOT_CONVERGED;
+    };
+    // the whole solve in one kernel: (r, p) pairs in the place of r and r0
+    const mcb::TeamMem team{(unsigned int *)(status + kArriveDouble), v.partials};
+    if (mcb::bicg_team(s, A, b, x, (double2 *)v.r, v.v[0], v.v[1], v.st, rtol, max_iters, team)) {
+        if (cudaMemcpyAsync(&hs, v.st, sizeof(hs), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MC_ERR_CUDA;
+        if (cudaStreamSynchronize(s) != cudaSuccess) return MC_ERR_CUDA;
+        return status_of();
+    }
     mcb::bicg_init<1>(s, A, v, rtol, max_iters);
     if (cudaGetLastError() != cudaSuccess) return MC_ERR_CUDA;
 
     constexpr int kBatch = 8;  // iterations between status reads (even: ping-pong buffers)
-    mcb::BicgState<1> hs{};
     const long max_batches = max_iters / kBatch + 2;
     for (long batch = 0;; batch++) {
         if (cudaMemcpyAsync(&hs, v.st, sizeof(hs), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MC_ERR_CUDA;
@@ -122,8 +137,5 @@ extern "C" int mc_solve_bicgstab_noalloc(int n, const double *diag, const double
         }
         if (cudaGetLastError() != cudaSuccess) return MC_ERR_CUDA;
     }
-    if (iterations) *iterations = hs.iter[0];
-    if (hs.status[0] == mcb::KRYLOV_NONFINITE) return MC_ERR_NONFINITE;
-    if (hs.status[0] != mcb::KRYLOV_OK) return MC_ERR_NOT_CONVERGED;
-    return MC_OK;
+    return status_of();
 }

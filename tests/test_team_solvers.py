@@ -1,0 +1,71 @@
+"""Krylov solves run as one kernel by a team of blocks (cluster up to 16 x 1024
+rows, then a cooperative grid with one or two rows per thread), at the edges
+of the team's forms: BiCGStab through the allocation-free entry point, its
+true residual checked in FP64 on the CPU, and the Jacobi-preconditioned
+pressure solve against the AMG-preconditioned one (the per-kernel solvers) on
+the same passes.
+
+Tolerances: BiCGStab stops on its recursive residual at 1e-10 ||b||, which
+stays within rounding of the true one on these diagonally dominant systems
+(checked at 2e-10).  Pressure solves run to 1e-12 of ||b||; two solutions then
+differ by at most 2e-12 times the condition number (below 1e4 at these sizes)
+relative to the correction, itself a small part of the fields: 1e-9.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+from minicombust_app_b200 import flow
+from minicombust_app_b200.workload import noisy_fields
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 31, 129, 1025, 2047, 2048, 9000, 16384, 16385, 151553, 262144])
+def test_bicgstab_team(gpu, n):
+    import torch
+    rng = np.random.default_rng(n)
+    idx = np.arange(n)
+    off, col = np.zeros((6, n)), np.tile(idx.astype(np.int32), (6, 1))
+    for k, d in enumerate((-700, -13, -1, 1, 13, 700)):
+        ok = (idx + d >= 0) & (idx + d < n)
+        off[k, ok] = -(0.2 + rng.random(int(ok.sum())))
+        col[k, ok] = (idx[ok] + d).astype(np.int32)
+    diag = 1.02 * np.abs(off).sum(axis=0) + 0.5
+    b = rng.standard_normal(n)
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (diag, off, col, b)]
+    L = flow.library()
+    for _ in range(2):  # the second call finds the first one's scratch
+        x = torch.full((n,), float("nan"), dtype=torch.float64, device="cuda")
+        its = ctypes.c_int(-1)
+        torch.cuda.synchronize()
+        rc = L.mc_solve_bicgstab_noalloc(n, *(t.data_ptr() for t in dev), x.data_ptr(), 1e-10, 500, None,
+                                         ctypes.byref(its))
+        assert rc == flow.MC_OK and its.value > 0
+        got = x.cpu().numpy()
+        res = b - diag * got - sum(off[k] * got[col[k]] for k in range(6))
+        assert np.linalg.norm(res) <= 2e-10 * np.linalg.norm(b)
+    rc = L.mc_solve_bicgstab_noalloc(n, *(t.data_ptr() for t in dev), x.data_ptr(), 1e-14, 1, None, None)
+    assert rc == (flow.MC_OK if n == 1 else flow.MC_ERR_NOT_CONVERGED)
+
+
+@pytest.mark.parametrize("dims,reorder", [((8, 4, 4), 0), ((17, 11, 11), 0), ((32, 32, 16), 0), ((33, 25, 20), 0),
+                                          ((33, 25, 20), 1), ((80, 44, 43), 0), ((80, 44, 44), 0)])
+def test_pcg_team_matches_amg(gpu, dims, reorder):
+    out = []
+    for psolver in (flow.PSOLVER_PCG_JACOBI, flow.PSOLVER_PCG_AMG):
+        s = flow.FlowSolver(flow.Mesh.box(*dims, 0.2, 0.1, 0.1),
+                            params=flow.default_params(flow.MODE_SIMPLE, pressure_solver=psolver, reorder=reorder,
+                                                       u_rtol=1e-12, p_rtol=1e-12))
+        for name, vals in noisy_fields(s.N, 5).items():
+            a = s.field(name)
+            a[:s.N] = vals
+            s.set_field(name, a)
+        for _ in range(2):
+            s.simple_iteration()
+        assert s.last_stats.pressure_rel_residual_first <= 1e-12
+        out.append({n: s.field(n) for n in ("U", "V", "W", "P", "TEM")})
+        s.close()
+    for n, a in out[0].items():
+        assert np.abs(a - out[1][n]).max() <= 1e-9 * np.abs(a).max(), n
