@@ -1733,7 +1733,7 @@ int setup_guess(mc_flow *h, const HostMesh &hm)
     const size_t N = (size_t)hm.N;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t eb = al(6 * N * 4), vb = al(N * 4), xb = al(N * 8), pb = al((size_t)GNN_NPARAM * 4),
-                 kb = al((size_t)GNN_NPACK * 2), wb = gnn_work_bytes(hm.N, false), mb = al(mask.size()),
+                 kb = al((size_t)GNN_NPACK * 2), wb = gnn_work_bytes(hm.N, 0), mb = al(mask.size()),
                  cb = al(6 * N * 4);
     const cudaError_t e = cudaMalloc((void **)&h->gnn_mem, eb + vb + xb + pb + kb + wb + mb + cb);
     if (e != cudaSuccess) return fail(h, MC_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
@@ -1750,7 +1750,7 @@ int setup_guess(mc_flow *h, const HostMesh &hm)
     h->gnn_p = reinterpret_cast<float *>(c + eb + vb + xb);
     h->gnn_pk = reinterpret_cast<__nv_bfloat16 *>(c + eb + vb + xb + pb);
     CUDA_TRY(h, cudaMemset(c + eb + vb + xb + pb + kb, 0, wb));
-    gnn_work_carve(h->gnn_w, c + eb + vb + xb + pb + kb, hm.N, false);
+    gnn_work_carve(h->gnn_w, c + eb + vb + xb + pb + kb, hm.N, 0);
     h->gnn_g.affine = aff.affine;
     for (int k = 0; k < 6; k++) {
         h->gnn_g.doff[k] = aff.doff[k];

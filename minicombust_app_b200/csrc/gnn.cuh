@@ -38,6 +38,7 @@ constexpr int GNN_H = 32;
 constexpr int GNN_L = 4;
 constexpr int GNN_IN = 4;
 constexpr int GNN_TILE = 128;   // cells per block
+constexpr int GNN_MAX_BATCH = 8;  // samples trained by one set of launches
 
 // Parameter layout (FP32 master copy, flat).
 constexpr int GP_WE = 0;                         // [H][IN]
@@ -102,7 +103,7 @@ struct GnnInput {
 // Device scratch for one graph size.
 struct GnnWork {
     int n = 0, nblocks = 0;
-    bool train = false;
+    int samples = 0;                     // training: samples the arrays hold, one after the other; 0: inference
     __nv_bfloat16 *h[GNN_L + 1] = {};   // activations [n][H]; inference uses h[0], h[1] as ping-pong
     __nv_bfloat16 *a[GNN_L] = {};       // training: relu(W1 u + c1) per layer
     __nv_bfloat16 *q = nullptr;          // training: decoder hidden
@@ -114,14 +115,17 @@ struct GnnWork {
     double *partials = nullptr;          // reductions
     unsigned int *counter = nullptr;
     GnnScales *scales = nullptr;
-    double *loss = nullptr;              // [2]: mean offset, loss
+    double *loss = nullptr;              // [samples][2]: mean offset, loss
     __nv_bfloat16 *fold = nullptr;       // [L][7][H][H] offset-form weights (inference)
     int *status = nullptr;               // nonzero: a tensor-core layer gave up waiting (prediction zeroed)
 };
 
-size_t gnn_work_bytes(int n, bool train);
-// Carve a work area out of `base` (gnn_work_bytes(n, train) bytes, 256-byte aligned).
-void gnn_work_carve(GnnWork &w, char *base, int n, bool train);
+size_t gnn_work_bytes(int n, int samples);
+// Carve a work area out of `base` (gnn_work_bytes(n, samples) bytes, 256-byte
+// aligned) for inference (samples 0) or the training of `samples` at a time.
+void gnn_work_carve(GnnWork &w, char *base, int n, int samples);
+// Samples to train together on a graph of n cells.
+int gnn_train_samples(int n);
 
 // Host: Kaiming-uniform initialisation (splitmix64 stream from `seed`).
 void gnn_init_params(float *p, uint64_t seed);
@@ -171,11 +175,12 @@ void gnn_layer_umma(cudaStream_t s, const GnnGraph &g, const GnnTmaMap &map, con
                     const __nv_bfloat16 *wf, const __nv_bfloat16 *pkl, const __nv_bfloat16 *hin,
                     __nv_bfloat16 *hout, int *status, int grid, const GnnUmmaDecode *dec = nullptr);
 
-// Training: forward, loss against `target` (units of the solution), backward;
-// adds this sample's gradient, scaled by `weight`, into grad[NPARAM] and
-// the sample's loss into w.loss[1] (overwritten).
-void gnn_loss_backward(cudaStream_t s, const GnnGraph &g, const GnnInput<float> &in, const float *target,
-                       const float *p, const __nv_bfloat16 *pk, GnnWork &w, float *grad, float weight);
+// Training: forward, loss against `target` (units of the solution), backward
+// of up to w.samples samples; adds their gradients, scaled by `weight`, into
+// grad[NPARAM] and writes sample q's loss to w.loss[2 q + 1].
+void gnn_loss_backward(cudaStream_t s, const GnnGraph &g, int samples, const GnnInput<float> *in,
+                       const float *const *target, const float *p, const __nv_bfloat16 *pk, GnnWork &w, float *grad,
+                       float weight);
 
 // Host: graph arrays of a solver mesh (its own numbering): direction-slot
 // columns, the per-slot face features as BF16 pairs, normalised volumes.

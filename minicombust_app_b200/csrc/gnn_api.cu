@@ -93,7 +93,7 @@ struct mc_gnn {
     char *work_mem = nullptr;
     size_t work_bytes = 0;
     GnnWork work;
-    double *h_loss = nullptr;  // pinned [2]
+    double *h_loss = nullptr;  // pinned [GNN_MAX_BATCH][2]
 };
 
 struct mc_gnn_graph {
@@ -120,10 +120,12 @@ int cuda_status(cudaError_t e) { return e == cudaSuccess ? MC_OK : (e == cudaErr
         if (rc_) return rc_;                   \
     } while (0)
 
-int ensure_work(mc_gnn *net, int n)
+// Work area for inference (samples 0) or training of `samples` at a time; a
+// training area also serves inference on the same graph size.
+int ensure_work(mc_gnn *net, int n, int samples)
 {
-    const size_t need = gnn_work_bytes(n, true);
-    if (net->work_mem && net->work.n == n) return MC_OK;
+    const size_t need = gnn_work_bytes(n, samples);
+    if (net->work_mem && net->work.n == n && net->work.samples >= samples) return MC_OK;
     if (net->work_mem) {
         cudaStreamSynchronize(net->stream);
         cudaFree(net->work_mem);
@@ -132,7 +134,7 @@ int ensure_work(mc_gnn *net, int n)
     GNN_TRY(cudaMalloc((void **)&net->work_mem, need));
     GNN_TRY(cudaMemsetAsync(net->work_mem, 0, need, net->stream));
     net->work_bytes = need;
-    gnn_work_carve(net->work, net->work_mem, n, true);
+    gnn_work_carve(net->work, net->work_mem, n, samples);
     return MC_OK;
 }
 
@@ -169,7 +171,7 @@ int mc_gnn_create(int device, uint64_t seed, mc_gnn **out)
         gnn_pack(net->stream, net->p, net->pk);
         rc = cuda_status(cudaGetLastError());
     }
-    if (!rc) rc = cuda_status(cudaMallocHost((void **)&net->h_loss, 2 * sizeof(double)));
+    if (!rc) rc = cuda_status(cudaMallocHost((void **)&net->h_loss, 2 * GNN_MAX_BATCH * sizeof(double)));
     if (!rc) rc = cuda_status(cudaStreamSynchronize(net->stream));
     if (rc) {
         mc_gnn_destroy(net);
@@ -286,7 +288,7 @@ int mc_gnn_predict(mc_gnn *net, const mc_gnn_graph *gr, const mc_gnn_sample *s, 
 {
     if (!net || !gr || !s || !s->rhs || !s->diag) return MC_ERR_ARG;
     GNN_TRY(cudaSetDevice(net->dev));
-    int rc = ensure_work(net, gr->g.n);
+    int rc = ensure_work(net, gr->g.n, 0);
     if (rc) return rc;
     gnn_forward<float>(net->stream, gr->g, input_of(*s), net->p, net->pk, net->work, x0);
     if (y) GNN_TRY(cudaMemcpyAsync(y, net->work.y, (size_t)gr->g.n * 4, cudaMemcpyDeviceToDevice, net->stream));
@@ -304,17 +306,25 @@ int mc_gnn_loss_grad(mc_gnn *net, const mc_gnn_graph *gr, int batch, const mc_gn
     for (int b = 0; b < batch; b++)
         if (!samples[b].rhs || !samples[b].diag || !samples[b].target) return MC_ERR_ARG;
     GNN_TRY(cudaSetDevice(net->dev));
-    int rc = ensure_work(net, gr->g.n);
+    int rc = ensure_work(net, gr->g.n, std::min(batch, gnn_train_samples(gr->g.n)));
     if (rc) return rc;
     GNN_TRY(cudaMemsetAsync(net->grad, 0, (size_t)GNN_NPARAM * 4, net->stream));
     double total = 0.0;
-    for (int b = 0; b < batch; b++) {
-        gnn_loss_backward(net->stream, gr->g, input_of(samples[b]), samples[b].target, net->p, net->pk, net->work,
-                          net->grad, 1.0f / batch);
+    for (int b = 0; b < batch;) {
+        const int q = std::min(batch - b, net->work.samples);
+        GnnInput<float> in[GNN_MAX_BATCH];
+        const float *target[GNN_MAX_BATCH];
+        for (int k = 0; k < q; k++) {
+            in[k] = input_of(samples[b + k]);
+            target[k] = samples[b + k].target;
+        }
+        gnn_loss_backward(net->stream, gr->g, q, in, target, net->p, net->pk, net->work, net->grad, 1.0f / batch);
         GNN_TRY(cudaGetLastError());
-        GNN_TRY(cudaMemcpyAsync(net->h_loss, net->work.loss, 2 * sizeof(double), cudaMemcpyDeviceToHost, net->stream));
+        GNN_TRY(cudaMemcpyAsync(net->h_loss, net->work.loss, 2 * q * sizeof(double), cudaMemcpyDeviceToHost,
+                                net->stream));
         GNN_TRY(cudaStreamSynchronize(net->stream));
-        total += net->h_loss[1];
+        for (int k = 0; k < q; k++) total += net->h_loss[2 * k + 1];
+        b += q;
     }
     if (loss) *loss = total / batch;
     if (host_grad) {
