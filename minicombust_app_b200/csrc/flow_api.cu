@@ -39,7 +39,7 @@ enum KernelId {
     K_BICG1_1, K_BICG1_2, K_BICG1_3, K_AMG_SETUP, K_PCG_INIT_AMG, K_PCG_ITER2_AMG, K_AMG_VCYCLE,
     K_IR, K_PCG_INIT_AMG32, K_PCG_ITER1_32, K_PCG_ITER2_AMG32, K_AMG_VCYCLE32, K_PERMUTE, K_GUESS, K_GNN,
     K_SNAPSHOT, K_BIR, K_ROUND_ELL, K_BICG3_INIT32, K_BICG3_1_32, K_BICG3_2_32, K_BICG3_3_32, K_BICG1_INIT32,
-    K_BICG1_1_32, K_BICG1_2_32, K_BICG1_3_32, K_GRAD6, K_SCALAR, K_SCALAR_CLIP, K_EXCHANGE, K_LINE3, K_LINE1,
+    K_BICG1_1_32, K_BICG1_2_32, K_BICG1_3_32, K_GRAD6, K_SCALAR, K_SCALAR_CLIP, K_EXCHANGE,
     K_GNN_LAYERS, K_SWEEP3, K_SWEEP1, K_PCG_TEAM, K_BICG1_TEAM, K_COUNT
 };
 
@@ -54,7 +54,7 @@ const char *kKernelNames[K_COUNT] = {
     "snapshot_pack", "bicg_refine_fp64_residual", "round_fp32", "bicg3_32_init", "bicg3_32_1_spmv",
     "bicg3_32_2_spmv", "bicg3_32_3_update", "bicg1_32_init", "bicg1_32_1_spmv", "bicg1_32_2_spmv",
     "bicg1_32_3_update", "lsq_gradients_scalars", "scalar_assemble", "scalar_clip_negative", "particle_exchange",
-    "line_sweep3_32", "line_sweep1_32", "gnn_layers", "line_sweep3_64", "line_sweep1_64",
+    "gnn_layers", "line_sweep3_64", "line_sweep1_64",
     "pcg_team", "bicg1_team"};
 
 constexpr int PCG_BATCH = 16;   // iterations per status read (even: ping-pong buffers)
@@ -172,12 +172,9 @@ struct mc_flow {
     BirState<1> *h_bo1 = nullptr;
     cudaGraphExec_t g_b3_32 = nullptr, g_b1_32 = nullptr;
     char *bir_mem = nullptr;
-    // x-line sweep inner solves (ir_line_steps > 0 on a box whose cells run
-    // x-fastest): line length, the two systems and a scratch iterate
+    // x-line sweeps (momentum, temperature, scalars) on a box whose cells run
+    // x-fastest: the line length, 0 where they do not
     int line_ex = 0;
-    LineSystem line3{}, line1{};
-    float *line_scratch = nullptr;
-    // the same lines for the FP64 sweeps (momentum, temperature, scalars)
     LineRows64 line64{};              // diag and off are set for each solve
     SweepState<3> *sweep3 = nullptr, *h_sweep3 = nullptr;  // device; pinned
     SweepState<1> *sweep1 = nullptr, *h_sweep1 = nullptr;
@@ -837,12 +834,22 @@ constexpr int SWEEP_MIN_ITERS = 50;
 // open system (a BiCGStab iteration moves four times a sweep's bytes and takes
 // about a decade off), or a non-finite value -- and the caller runs BiCGStab
 // from zero.
+// With FP32 refinement the sweeps are used unless ir_line_steps asks for the
+// inner BiCGStab: in FP64 they move 448 bytes per row for the three momentum
+// systems, fewer than FP32 sweeps with an FP64 residual after each pair
+// (2 x 128^3, ms per pass: momentum 0.64 -> 0.50, temperature 0.34 -> 0.31, each
+// assembly 0.02 less without the FP32 rows), and their errors are 100 times smaller.
+bool sweeps_apply(const mc_flow *h)
+{
+    return h->line_ex > 0 && h->prm.max_iters >= SWEEP_MIN_ITERS && (!h->bir_mem || h->prm.ir_line_steps > 0);
+}
+
 template <int R>
 int solve_sweeps(mc_flow *h, const double *diag, const double *off, const double *b, double *const (&x)[R],
                  double *scratch, SweepState<R> *st, SweepState<R> *hs, int iters_out[R], bool *used)
 {
     *used = false;
-    if (h->line_ex == 0 || h->prm.max_iters < SWEEP_MIN_ITERS) return MC_OK;
+    if (!sweeps_apply(h)) return MC_OK;
     LineRows64 L = h->line64;
     L.diag = diag;
     L.off = off;
@@ -890,8 +897,6 @@ int solve_bicg_refined(mc_flow *h, const Ell &A, const EllT<float> &A32, const B
                        cudaGraphExec_t *loop, int kid_init32, int kid1_32, int iters_out[R])
 {
     constexpr int kMaxOuter = 30;
-    const LineSystem *line = nullptr;
-    if (h->prm.ir_line_steps > 0 && h->line_ex > 0) line = (R == 3) ? &h->line3 : &h->line1;
     launch(h, K_BIR, [&] { bir_init<R>(h->stream, A, out, h->prm.u_rtol, kMaxOuter); });
     int rc = check_launch(h);
     if (rc) return rc;
@@ -923,32 +928,6 @@ int solve_bicg_refined(mc_flow *h, const Ell &A, const EllT<float> &A32, const B
         }
         if (hout->all_done) break;
         if (outer > kMaxOuter) return fail(h, MC_ERR_NOT_CONVERGED, "refinement state did not advance");
-        if (line) {
-            // x-line sweep steps on the row-scaled FP32 system; the last step
-            // writes the inner solution out.e.  A step reduces the residual by
-            // about 10^3 on the flows this is meant for, so when every open
-            // system is within 10^3 of its tolerance one step is taken (a slower
-            // step only costs another outer iteration)
-            double need = 1.0;
-            for (int j = 0; j < R; j++)
-                if (!hout->done[j] && hout->rr[j] > 0) need = std::min(need, std::sqrt(hout->tol2[j] / hout->rr[j]));
-            const int K = need >= 1e-3 ? 1 : h->prm.ir_line_steps;
-            float *E[2] = {const_cast<float *>(out.e), h->line_scratch};
-            // the last step adds its result to x (the refinement update)
-            for (int k = 1; k <= K; k++) {
-                float *dst = E[(K - k) % 2];
-                const float *prev = E[(K - k + 1) % 2];
-                launch(h, R == 3 ? K_LINE3 : K_LINE1, [&] {
-                    line_step<R>(h->stream, *line, out.r32, prev, dst, k == 1 ? 1 : 0, k == K ? &out : nullptr);
-                });
-            }
-            for (int j = 0; j < R; j++)
-                if (!hout->done[j]) iters_out[j] += K;
-            launch(h, K_BIR, [&] { bir_residual<R>(h->stream, A, out); });
-            rc = check_launch(h);
-            if (rc) return rc;
-            continue;
-        }
         double inner_rtol = 0.5;
         for (int j = 0; j < R; j++)
             if (!hout->done[j] && hout->rr[j] > 0)
@@ -1186,13 +1165,14 @@ int stage_momentum(mc_flow *h, mc_iter_stats *st)
     a.store = h->rows;
     a.AU = h->AU;
     a.b = h->b_m;
-    const bool fused32 = h->bir_mem && h->dc.code;  // the FP32 copy written by the assembly itself
+    const bool lines = sweeps_apply(h);
+    const bool fused32 = h->bir_mem && !lines && h->dc.code;  // the FP32 copy written by the assembly itself
     if (fused32) a.f32 = Fp32Rows{h->m32_diag, h->m32_off, h->dc.code};
     launch(h, K_MOMENTUM, [&] { k_momentum_assemble<<<blocks_for(h->N), MCB_THREADS, 0, h->stream>>>(h->ph, h->margs, a); });
     int rc = check_launch(h);
     if (rc) return rc;
     int its[3] = {0, 0, 0};
-    if (h->bir_mem) {
+    if (h->bir_mem && !lines) {
         if (!fused32)
             launch(h, K_ROUND_ELL,
                    [&] { round_ell(h->stream, h->N, h->AU, h->off_m, h->dc.code, h->m32_diag, h->m32_off); });
@@ -1350,7 +1330,8 @@ int stage_temperature(mc_flow *h, mc_iter_stats *st)
     a.b = h->b_t;
     a.imbalance = h->scalars + 1;
     CUDA_TRY(h, cudaMemsetAsync(a.imbalance, 0, sizeof(double), h->stream));
-    const bool fused32 = h->bir_mem && h->dc.code;
+    const bool lines = sweeps_apply(h);
+    const bool fused32 = h->bir_mem && !lines && h->dc.code;
     if (fused32) a.f32 = Fp32Rows{h->t32_diag, h->t32_off, h->dc.code};
     launch(h, K_TEMPERATURE, [&] {
         k_temperature_assemble<<<blocks_for(h->N), MCB_THREADS, 0, h->stream>>>(h->ph, h->margs, a);
@@ -1358,7 +1339,7 @@ int stage_temperature(mc_flow *h, mc_iter_stats *st)
     int rc = check_launch(h);
     if (rc) return rc;
     int its[1] = {0};
-    if (h->bir_mem) {
+    if (h->bir_mem && !lines) {
         if (!fused32)
             launch(h, K_ROUND_ELL,
                    [&] { round_ell(h->stream, h->N, h->diag_t, h->off_t, h->dc.code, h->t32_diag, h->t32_off); });
@@ -1685,31 +1666,6 @@ int setup_bicg_refined(mc_flow *h)
     h->bo3 = BirVectors<3>{{h->phi[G_U], h->phi[G_V], h->phi[G_W]}, h->b_m, vec[1], vec[0], h->partials, h->counter,
                            bo3};
     h->bo1 = BirVectors<1>{{h->phi[G_T]}, h->b_t, vec[1], vec[0], h->partials, h->counter, bo1};
-    if (h->line_ex > 0) {
-        // the FP32 copies are stored by direction: slot d holds direction d
-        LineSystem L;
-        L.N = h->N;
-        L.ex = h->line_ex;
-        int q = 0;
-        for (int d = 0; d < 6; d++) {
-            if (h->dc.doff[d] == -1)
-                L.dxm = d;
-            else if (h->dc.doff[d] == 1)
-                L.dxp = d;
-            else {
-                L.yz[q] = d;
-                L.yzoff[q] = h->dc.doff[d];
-                q++;
-            }
-        }
-        h->line3 = L;
-        h->line3.d = h->m32_diag;
-        h->line3.off = h->m32_off;
-        h->line1 = L;
-        h->line1.d = h->t32_diag;
-        h->line1.off = h->t32_off;
-        h->line_scratch = vec[2];  // the inner BiCGStab's r, unused by the line solver
-    }
     CUDA_TRY(h, cudaMallocHost((void **)&h->h_bi3, sizeof(BicgState<3>)));
     CUDA_TRY(h, cudaMallocHost((void **)&h->h_bi1, sizeof(BicgState<1>)));
     CUDA_TRY(h, cudaMallocHost((void **)&h->h_bo3, sizeof(BirState<3>)));

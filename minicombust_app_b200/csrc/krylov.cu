@@ -1162,136 +1162,17 @@ void bir_residual(cudaStream_t s, const Ell &A, const BirVectors<R> &v)
 {
     k_bir_residual<R><<<krylov_grid(A.N), MCB_THREADS, 0, s>>>(A, v);
 }
-// ------------------------------------------------------- x-line sweeps
+// ---------------------------------------------------- FP64 x-line sweeps
 //
 // Splitting A = M - (M - A) with M the diagonal and the -x couplings of each
 // x-line (a lower bidiagonal block per line: the upwind direction of the
-// x-directed flow): one step solves M e_new = r - (M - A) e_prev, i.e. the
+// x-directed flow): one sweep solves M x_{k+1} = b - (A - M) x_k, i.e. the
 // +x, y and z couplings of the previous iterate go to the right-hand side
-// and each line is a first-order recurrence e_k = (rhs_k - a_k e_{k-1}) / b_k.
-// A is an M-matrix (positive diagonal, non-positive couplings, diagonally
-// dominant through the transient term), so this is a regular splitting and
-// the iteration converges; with convection along +x the neglected couplings
-// are small and each step reduces the residual by orders of magnitude.
-//
-// One warp per line.  First every cell's affine map e_k = p_k + q_k e_{k-1}
-// is formed from coalesced loads (32 consecutive cells per step, all of the
-// line's loads independent, so they overlap) and kept in shared memory; then
-// the warp walks the line in chunks of 32: a warp scan (shuffles) composes
-// the chunk's maps, the value entering the chunk is applied, and the chunk's
-// last value is carried into the next chunk.
-template <int R>
-struct LineAdd {
-    double *x[R];
-    const BirState<R> *st = nullptr;  // null: store e_new
-};
-
-template <int R>
-__global__ void __launch_bounds__(256, R == 1 ? 8 : 6) k_line_sweep(LineSystem L, const float *__restrict__ r,
-                                                    const float *__restrict__ ep, float *__restrict__ en, int first,
-                                                    LineAdd<R> add)
-{
-    extern __shared__ float sline[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int line = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int N = L.N, ex = L.ex;
-    if (line >= N / ex) return;
-    float *sq = sline + (size_t)warp * ex * (R + 1);  // q[ex], then p[R][ex]
-    float *sp = sq + ex;
-    const size_t base = (size_t)line * ex;
-#pragma unroll 1
-    for (int c = lane; c < ex; c += 32) {
-        const size_t i = base + c;
-        const float a = L.off[(size_t)L.dxm * N + i];
-        const float b = L.d[i];
-        float rhs[R];
-#pragma unroll
-        for (int j = 0; j < R; j++) rhs[j] = r[(size_t)j * N + i];
-        if (!first) {
-            if (c + 1 < ex) {
-                const float o = L.off[(size_t)L.dxp * N + i];
-#pragma unroll
-                for (int j = 0; j < R; j++) rhs[j] -= o * ep[(size_t)j * N + i + 1];
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const float o = L.off[(size_t)L.yz[u] * N + i];
-                const long nb = min(max((long)i + L.yzoff[u], 0L), (long)N - 1);
-#pragma unroll
-                for (int j = 0; j < R; j++) rhs[j] -= o * ep[(size_t)j * N + nb];
-            }
-        }
-        const float rb = 1.f / b;
-        sq[c] = -a * rb;
-#pragma unroll
-        for (int j = 0; j < R; j++) sp[j * ex + c] = rhs[j] * rb;
-    }
-    __syncwarp();
-    bool act[R];
-#pragma unroll
-    for (int j = 0; j < R; j++) act[j] = add.st && !add.st->done[j];
-    float carry[R];
-#pragma unroll
-    for (int j = 0; j < R; j++) carry[j] = 0.f;
-    for (int c0 = 0; c0 < ex; c0 += 32) {
-        const int c = c0 + lane;
-        float p[R], q = 1.f;
-#pragma unroll
-        for (int j = 0; j < R; j++) p[j] = 0.f;
-        if (c < ex) {
-            q = sq[c];
-#pragma unroll
-            for (int j = 0; j < R; j++) p[j] = sp[j * ex + c];
-        }
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            float pu[R];
-#pragma unroll
-            for (int j = 0; j < R; j++) pu[j] = __shfl_up_sync(0xffffffffu, p[j], off);
-            const float qu = __shfl_up_sync(0xffffffffu, q, off);
-            if (lane >= off) {
-#pragma unroll
-                for (int j = 0; j < R; j++) p[j] = p[j] + q * pu[j];
-                q = q * qu;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < R; j++) {
-            const float x = p[j] + q * carry[j];
-            if (c < ex) {
-                if (!add.st)
-                    en[(size_t)j * N + base + c] = x;
-                else if (act[j])
-                    add.x[j][base + c] += (double)x;
-            }
-            carry[j] = __shfl_sync(0xffffffffu, x, 31);
-        }
-    }
-}
-
-template <int R>
-void line_step(cudaStream_t s, const LineSystem &L, const float *r, const float *e_prev, float *e_new, int first,
-               const BirVectors<R> *add)
-{
-    LineAdd<R> la{};
-    if (add) {
-        for (int j = 0; j < R; j++) la.x[j] = add->x[j];
-        la.st = add->st;
-    }
-    const int lines = L.N / L.ex;
-    const size_t per_warp = (size_t)L.ex * (R + 1) * sizeof(float);
-    int warps = 8;
-    while (warps > 1 && warps * per_warp > 48 * 1024) warps >>= 1;
-    const int threads = 32 * warps;
-    const int grid = (lines + warps - 1) / warps;
-    k_line_sweep<R><<<grid, threads, warps * per_warp, s>>>(L, r, e_prev, e_new, first, la);
-}
-template void line_step<1>(cudaStream_t, const LineSystem &, const float *, const float *, float *, int,
-                           const BirVectors<1> *);
-template void line_step<3>(cudaStream_t, const LineSystem &, const float *, const float *, float *, int,
-                           const BirVectors<3> *);
-
-// ---------------------------------------------------- FP64 x-line sweeps
+// and each line is a first-order recurrence.  A is an M-matrix (positive
+// diagonal, non-positive couplings, diagonally dominant through the transient
+// term), so this is a regular splitting and converges; with convection along +x
+// the neglected couplings are small and each sweep takes the residual down by
+// about three decades.
 //
 // HBM bound: a sweep streams the row once for all R systems, 56 bytes of
 // matrix and per system b, x_k and x_{k+1} (24 bytes; 16 for the first sweep,
@@ -1299,12 +1180,17 @@ template void line_step<3>(cudaStream_t, const LineSystem &, const float *, cons
 // takes four sweeps, 448 bytes per row, where BiCGStab takes 8 to 10
 // iterations of 520: a plain FP64 timestep of the 2 x 128^3 box 48.6 -> 26.8 ms,
 // with errors against 64-bit solves ten times smaller.
-// One warp per line: the cells' affine maps e_i = p_i + q_i e_{i-1} are formed
-// from independent coalesced loads into shared memory, then composed by warp
-// scans of 32 cells and a carry.  The residual of the iterate read is the
-// right-hand side the map is formed from less its own diagonal and -x terms,
-// so convergence costs no extra pass over the matrix; the iterate returned is
-// one sweep better than the one tested.
+// One warp per line and system, the R warps of a line in one block (the matrix
+// comes from HBM once and from L1 for the others): 14 loads of 256 bytes in
+// flight per warp at 48 to 56 registers, 36 to 40 warps per SM.  Chunks of 32 cells: the
+// cells' affine maps e_i = p_i + q_i e_{i-1} from coalesced loads, a warp scan
+// composes them, the value entering the chunk is applied and its last value
+// carried on.  (All three systems in one warp, maps staged in shared memory,
+// held 24 warps per SM: a momentum solve's sweeps 0.63 ms at 2 x 128^3, in this
+// form 0.50 ms; 40 registers spill and take 0.62, 64 and 72 take 0.54.)
+// The residual of the iterate read is the right-hand side the map is formed
+// from less its own diagonal and -x terms, so convergence costs no extra pass
+// over the matrix; the iterate returned is one sweep better than the one tested.
 template <int R, bool DIR>
 __device__ __forceinline__ double line_value(const LineRows64 &L, size_t i, uint32_t cw, int d)
 {
@@ -1322,108 +1208,79 @@ struct SweepPtrs {
     double *out[R];
 };
 
-// Resident blocks of 256 per SM: 3 x 64 KB of maps for three systems (24
-// warps hold about 160 KB of loads in flight per SM), 4 for one.
+// Lines of a block, and blocks per SM.
 template <int R>
-constexpr int sweep_blocks() { return R == 1 ? 4 : 3; }
+constexpr int sweep_lines = R == 1 ? 8 : 3;
+template <int R>
+constexpr int sweep_blocks = R == 1 ? 5 : 4;
 
 template <int R, bool DIR, bool FIRST>
-__global__ void __launch_bounds__(256, sweep_blocks<R>())
+__global__ void __launch_bounds__(32 * R * sweep_lines<R>, sweep_blocks<R>)
     k_line_sweep64(LineRows64 L, SweepVectors<R> v, SweepPtrs<R> x, int to, double rtol)
 {
     pdl_wait();
-    extern __shared__ double sweep_smem[];
+    constexpr int LB = sweep_lines<R>;
     __shared__ double sw[R][32];
     SweepState<R> *st = v.st;
     if (!FIRST && st->all_done) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = warp % R;
     const int N = L.N, ex = L.ex, lines = N / ex;
-    double *sq = sweep_smem + (size_t)warp * ex * (R + 1);  // q[ex], then p[R][ex]
-    double *sp = sq + ex;
-    double acc[R];
-#pragma unroll
-    for (int j = 0; j < R; j++) acc[j] = 0.0;
-    for (int line = blockIdx.x * nw + warp; line < lines; line += gridDim.x * nw) {
-        const size_t base = (size_t)line * ex;
-#pragma unroll 1
-        for (int c = lane; c < ex; c += 32) {
-            const size_t i = base + c;
+    const double *__restrict__ xin = pick(x.in, j);
+    double *__restrict__ xout = pick(x.out, j);
+    const double *__restrict__ b = v.b + (size_t)j * N;
+    double sum = 0.0;
+    for (int line = blockIdx.x * LB + warp / R; line < lines; line += gridDim.x * LB) {
+        const int base = line * ex;
+        double carry = 0.0, xlast = 0.0;  // e and x of the cell before the chunk
+        for (int c0 = 0; c0 < ex; c0 += 32) {
+            const int c = c0 + lane, i = base + min(c, ex - 1);
+            const bool on = c < ex;
             const uint32_t cw = DIR ? 0u : L.code[i];
             const double d = L.diag[i];
             const double a = line_value<R, DIR>(L, i, cw, L.xm);
-            double rhs[R];
-#pragma unroll
-            for (int j = 0; j < R; j++) rhs[j] = v.b[(size_t)j * N + i];
+            double s = b[i];
             if (FIRST) {
-#pragma unroll
-                for (int j = 0; j < R; j++) acc[j] += rhs[j] * rhs[j];
+                if (on) sum += s * s;
             } else {
+                const double x0 = xin[i];
+                double xe = 0.0;  // the cell after the chunk's last
+                if (lane == 31 && c + 1 < ex) xe = xin[i + 1];
                 const double op = line_value<R, DIR>(L, i, cw, L.xp);
-                double oy[4];
-                size_t nb[4];
+                double o[4], xy[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    oy[u] = line_value<R, DIR>(L, i, cw, L.yz[u]);
-                    nb[u] = (size_t)min(max((long)i + L.yzoff[u], 0L), (long)N - 1);
+                    o[u] = line_value<R, DIR>(L, i, cw, L.yz[u]);
+                    xy[u] = xin[min(max(i + L.yzoff[u], 0), N - 1)];
                 }
-                const size_t im = c > 0 ? i - 1 : i, ip = c + 1 < ex ? i + 1 : i;
+                double xp = __shfl_down_sync(0xffffffffu, x0, 1), xm = __shfl_up_sync(0xffffffffu, x0, 1);
+                if (lane == 31) xp = xe;
+                if (lane == 0) xm = xlast;
+                xlast = __shfl_sync(0xffffffffu, x0, 31);
+                if (c + 1 < ex) s -= op * xp;
 #pragma unroll
-                for (int j = 0; j < R; j++) {
-                    const double *__restrict__ xin = x.in[j];
-                    const double x0 = xin[i], xm = xin[im], xp = xin[ip];
-                    double xy[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) xy[u] = xin[nb[u]];
-                    double s = rhs[j];
-                    if (c + 1 < ex) s -= op * xp;
-#pragma unroll
-                    for (int u = 0; u < 4; u++) s -= oy[u] * xy[u];
-                    rhs[j] = s;
-                    double res = s - d * x0;
-                    if (c > 0) res -= a * xm;
-                    acc[j] += res * res;
-                }
+                for (int u = 0; u < 4; u++) s -= o[u] * xy[u];
+                double res = s - d * x0;
+                if (c > 0) res -= a * xm;
+                if (on) sum += res * res;
             }
             const double rb = 1.0 / d;
-            sq[c] = -a * rb;
+            double p = on ? s * rb : 0.0, q = on ? -a * rb : 1.0;
 #pragma unroll
-            for (int j = 0; j < R; j++) sp[j * ex + c] = rhs[j] * rb;
-        }
-        __syncwarp();
-        double carry[R];
-#pragma unroll
-        for (int j = 0; j < R; j++) carry[j] = 0.0;
-        for (int c0 = 0; c0 < ex; c0 += 32) {
-            const int c = c0 + lane;
-            double p[R], q = 1.0;
-#pragma unroll
-            for (int j = 0; j < R; j++) p[j] = 0.0;
-            if (c < ex) {
-                q = sq[c];
-#pragma unroll
-                for (int j = 0; j < R; j++) p[j] = sp[j * ex + c];
-            }
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                double pu[R];
-#pragma unroll
-                for (int j = 0; j < R; j++) pu[j] = __shfl_up_sync(0xffffffffu, p[j], o);
-                const double qu = __shfl_up_sync(0xffffffffu, q, o);
-                if (lane >= o) {
-#pragma unroll
-                    for (int j = 0; j < R; j++) p[j] += q * pu[j];
+            for (int off = 1; off < 32; off <<= 1) {
+                const double pu = __shfl_up_sync(0xffffffffu, p, off), qu = __shfl_up_sync(0xffffffffu, q, off);
+                if (lane >= off) {
+                    p += q * pu;
                     q *= qu;
                 }
             }
-#pragma unroll
-            for (int j = 0; j < R; j++) {
-                const double e = p[j] + q * carry[j];
-                if (c < ex) x.out[j][base + c] = e;
-                carry[j] = __shfl_sync(0xffffffffu, e, 31);
-            }
+            const double e = p + q * carry;
+            if (on) xout[i] = e;
+            carry = __shfl_sync(0xffffffffu, e, 31);
         }
-        __syncwarp();  // the maps are read before the next line's replace them
     }
+    double acc[R];
+#pragma unroll
+    for (int q = 0; q < R; q++) acc[q] = q == j ? sum : 0.0;
     if (publish_sums<R>(acc, v.partials, v.counter, sw)) {
         double tot[R];
         reduce_sums<R>(tot, v.partials, v.counter, sw);
@@ -1454,26 +1311,19 @@ __global__ void __launch_bounds__(256, sweep_blocks<R>())
 }
 
 namespace {
-// Dynamic shared memory the sweeps may take: three blocks of it fit an SM.
-constexpr size_t SWEEP_SMEM_MAX = 72 * 1024;
-
 template <int R, bool DIR, bool FIRST>
 void launch_line_sweep64(cudaStream_t s, const LineRows64 &L, const SweepVectors<R> &v, int from, double rtol)
 {
-    const size_t per_warp = (size_t)L.ex * (R + 1) * sizeof(double);
-    int warps = 8;
-    while (warps > 1 && warps * per_warp > SWEEP_SMEM_MAX) warps >>= 1;
-    auto k = k_line_sweep64<R, DIR, FIRST>;
-    // (a per-device attribute of the function; setting it again costs nothing)
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SWEEP_SMEM_MAX);
+    constexpr int LB = sweep_lines<R>;
     const int lines = L.N / L.ex;
-    const int grid = std::min({(lines + warps - 1) / warps, line_sweep64_blocks(L.N), krylov_sms() * sweep_blocks<R>()});
+    const int grid =
+        std::min({(lines + LB - 1) / LB, line_sweep64_blocks(L.N), krylov_sms() * sweep_blocks<R>});
     SweepPtrs<R> x{};
     for (int j = 0; j < R; j++) {
         x.in[j] = v.x[from][j];
         x.out[j] = v.x[from ^ 1][j];
     }
-    pdl_launch(k, dim3(grid), dim3(32 * warps), warps * per_warp, s, L, v, x, from ^ 1, rtol);
+    pdl_launch(k_line_sweep64<R, DIR, FIRST>, dim3(grid), dim3(32 * R * LB), 0, s, L, v, x, from ^ 1, rtol);
 }
 } // namespace
 

@@ -269,30 +269,6 @@ struct BirVectors {
     BirState<R> *st;
 };
 
-// x-line sweeps: the inner solver of the refined momentum and temperature
-// systems (FP32, row-scaled, values by direction) on a structured box whose
-// cells run x-fastest along whole lines.  The splitting keeps, per x-line,
-// the diagonal and the -x couplings (a first-order recurrence along the
-// line); the other couplings act through the previous iterate.
-struct LineSystem {
-    int N = 0;
-    int ex = 0;        // cells per x-line (the line length, <= 1024)
-    int P = 0;         // unused (kept 0)
-    int dxm = 0, dxp = 0;      // by-direction slots of the -x and +x couplings
-    int yz[4] = {0, 0, 0, 0};  // the other four slots
-    int yzoff[4] = {0, 0, 0, 0};
-    const float *d = nullptr;   // diagonal [N]
-    const float *off = nullptr; // [6][N] by direction
-};
-// One sweep step for R right-hand sides [R][N]: with first set, M e_new = r;
-// otherwise M e_new = r - (M - A) e_prev.  With add set (the last step of an
-// inner solve) the step's result is added to the FP64 solutions add->x of
-// the systems still open instead of being stored (e_new unused): the
-// refinement update x += e without a kernel of its own.
-template <int R>
-void line_step(cudaStream_t s, const LineSystem &L, const float *r, const float *e_prev, float *e_new, int first,
-               const BirVectors<R> *add = nullptr);
-
 // FP64 x-line sweeps: the whole momentum or transport solve as the splitting
 // iteration x_{k+1} = M^-1 (b - (A - M) x_k), M the diagonal and the -x
 // couplings of each x-line, from x_0 = 0, on a structured box whose cells run
