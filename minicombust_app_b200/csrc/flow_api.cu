@@ -60,6 +60,7 @@ const char *kKernelNames[K_COUNT] = {
 constexpr int PCG_BATCH = 16;   // iterations per status read (even: ping-pong buffers)
 constexpr int PCG_AMG_BATCH = 4;
 constexpr int BICG_BATCH = 8;
+constexpr int IR_MAX_OUTER = 50;  // outer iterations of a refined pressure solve
 
 // One cudaMalloc carved into aligned sub-buffers.
 struct Arena {
@@ -150,6 +151,11 @@ struct mc_flow {
     cudaGraphExec_t l_pcg = nullptr, l_b3 = nullptr, l_b1 = nullptr, l_pcg_amg = nullptr;
     cudaGraphExec_t l_pcg_amg32 = nullptr, l_b3_32 = nullptr, l_b1_32 = nullptr;
     bool loops_failed = false;   // a loop graph could not be built: host-driven batches
+    // the first corrector of a pass as one graph (corrector_graph), the streams
+    // its loop bodies are captured on
+    cudaGraphExec_t g_corr = nullptr;
+    bool corr_failed = false;
+    cudaStream_t cap[2] = {nullptr, nullptr};
     // aggregation AMG (pressure_solver == MC_PSOLVER_PCG_AMG)
     bool use_amg = false;
     AmgHierarchy amg;
@@ -473,6 +479,43 @@ long loop_launches(int iters, int per_iter)
     return 1 + bodies * (LOOP_ITERS * per_iter + 1);
 }
 
+// While h->stream captures a graph: a test of *done and a conditional WHILE
+// node that repeats `body` until it is set, as in run_loop; loops nest (depth 0,
+// then 1).  The body is captured on h->cap[depth], which h->stream stands for
+// meanwhile.  False when a call failed (the capture is then abandoned).
+template <typename Body>
+bool capture_loop(mc_flow *h, int depth, const int *done, Body &&body)
+{
+    const cudaStream_t s = h->stream, b = h->cap[depth];
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaGraph_t g = nullptr;
+    const cudaGraphNode_t *deps = nullptr;
+    size_t nd = 0;
+    bool ok = cudaStreamGetCaptureInfo(s, &status, nullptr, &g) == cudaSuccess && g;
+    cudaGraphConditionalHandle hc{};
+    ok = ok && cudaGraphConditionalHandleCreate(&hc, g, 0, 0) == cudaSuccess;
+    if (!ok) return false;
+    k_loop_continue<<<1, 1, 0, s>>>(hc, done);
+    ok = cudaStreamGetCaptureInfo(s, &status, nullptr, &g, &deps, &nd) == cudaSuccess;
+    cudaGraphNodeParams cp{};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = hc;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    cudaGraphNode_t loop = nullptr;
+    ok = ok && cudaGraphAddNode(&loop, g, deps, nd, &cp) == cudaSuccess;
+    ok = ok && cudaStreamUpdateCaptureDependencies(s, &loop, 1, cudaStreamSetCaptureDependencies) == cudaSuccess;
+    ok = ok && cudaStreamBeginCaptureToGraph(b, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                             cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    if (!ok) return false;
+    h->stream = b;
+    const bool inner = body();
+    k_loop_continue<<<1, 1, 0, b>>>(hc, done);
+    h->stream = s;
+    cudaGraph_t captured = nullptr;
+    return cudaStreamEndCapture(b, &captured) == cudaSuccess && inner;
+}
+
 // Snapshot record [4][N] float32 in the caller's numbering (idx = old -> new
 // or nullptr): b - mean, diagonal, previous correction, correction.
 __global__ void k_snapshot_pack(int N, const double *__restrict__ b, const PcgState *__restrict__ st,
@@ -527,9 +570,10 @@ int select_guess(mc_flow *h, const Ell &A, const double *b, const PcgState *st, 
     return 1;
 }
 
-// After a solve: append a snapshot record, then keep the correction as the
+// After a solve from a guess: what the selection chose.
+// after_pressure_solve: also append a snapshot record, then keep the correction as the
 // next solve's previous correction.
-int after_pressure_solve(mc_flow *h)
+int check_guess(mc_flow *h)
 {
     if (h->prm.initial_guess != MC_GUESS_ZERO && h->corrector == 1) {
         const GuessState &g = *h->h_gs;  // the copy was ordered before the solve's final synchronisation
@@ -538,6 +582,12 @@ int after_pressure_solve(mc_flow *h)
         h->guess_choice = g.choice;
         h->guess_rel = g.bb > 0 ? std::sqrt((g.choice < 0 ? g.bb : g.rc) / g.bb) : 1.0;
     }
+    return MC_OK;
+}
+
+int after_pressure_solve(mc_flow *h)
+{
+    if (const int rg = check_guess(h)) return rg;
     if (h->snap && h->snap_count < h->snap_max) {
         launch(h, K_SNAPSHOT, [&] {
             k_snapshot_pack<<<blocks_for(h->N), MCB_THREADS, 0, h->stream>>>(
@@ -655,7 +705,7 @@ int solve_pressure_refined(mc_flow *h, double abs_floor, int *iters, double *rel
     const EllT<float> A32{h->N, h->amg.lv32[0].diag, h->amg.lv32[0].off, h->col, h->amg.lv32[0].dc};
     PcgVectors o = h->pv;
     PcgVectorsT<float> in = h->pv32;
-    constexpr int kMaxOuter = 50;
+    constexpr int kMaxOuter = IR_MAX_OUTER;
     launch(h, K_PCG_MEAN, [&] { pcg_mean(h->stream, A, o); });
     const int use_x0 = select_guess(h, A, o.b, o.st, o.x, true);
     h->guess_used = use_x0 != 0;
@@ -1043,6 +1093,119 @@ void launch_mass_flux(mc_flow *h)
         });
 }
 
+// The corrections of one corrector: the correction's gradient, the face
+// fluxes, then the cells (with the next corrector's right-hand side in simple mode).
+void launch_corrections(mc_flow *h, int simple, int cell0)
+{
+    launch_gradient_pressure(h, G_PP);
+    CorrectArgs c{};
+    c.PP = h->phi[G_PP];
+    c.P = h->phi[G_P];
+    c.U = h->phi[G_U];
+    c.V = h->phi[G_V];
+    c.W = h->phi[G_W];
+    c.AU = h->AU;
+    for (int d = 0; d < 3; d++) c.gPP[d] = h->grad[G_PP][d];
+    c.ff0 = h->ff0;
+    c.mdot = h->mdot;
+    c.fcorr = h->fcorr;
+    c.next_rhs = simple ? h->b_p : nullptr;
+    c.rhs_max = simple ? h->scalars + 4 : nullptr;
+    const int grid_f = std::min(blocks_for(h->F), krylov_grid(h->F));
+    launch(h, K_PP_FACES, [&] { k_pp_correct_faces<<<grid_f, MCB_THREADS, 0, h->stream>>>(h->ph, h->margs, c); });
+    launch(h, K_PP_CELLS, [&] {
+        k_pp_correct_cells<<<blocks_for(h->N + 6), MCB_THREADS, 0, h->stream>>>(h->ph, h->margs, c, simple, cell0);
+    });
+}
+
+// The first corrector of a simple-mode pass with AMG, from the solve's
+// initialisation to the corrections, as one graph: the solve's loops run on the
+// device (the refinement's outer loop too, its inner tolerances formed there)
+// and the host waits once, after the corrections, instead of once per outer
+// iteration and once for the largest correction; the launches cost the device
+// about 1 us each instead of the host's 2 to 3.  Below a million cells this is
+// what a pass waits for (timestep, before and after: 1k cells 1.50 -> 1.28 ms, 65k
+// 3.18 -> 2.95, 305k refined 5.11 -> 4.79, 524k 8.57 -> 8.29).
+// False (nothing launched) when the graph cannot be built.
+bool corrector_graph(mc_flow *h, int use_x0)
+{
+    if (!use_loops(h) || h->corr_failed || !h->use_amg || h->prm.mode != MC_MODE_SIMPLE || h->snap) return false;
+    if (!h->g_corr) {
+        bool ok = true;
+        for (cudaStream_t &c : h->cap)
+            if (!c) ok = ok && cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking) == cudaSuccess;
+        ok = ok && cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+        if (ok) {
+            const long before = h->launches;
+            const Ell A = pressure_matrix(h);
+            const PcgVectors v = h->pv;
+            const double *x2 = nullptr;
+            if (h->refined) {
+                const EllT<float> A32{h->N, h->amg.lv32[0].diag, h->amg.lv32[0].off, h->col, h->amg.lv32[0].dc};
+                const PcgVectorsT<float> in = h->pv32;
+                IrGuess g{};
+                if (use_x0)
+                    g = IrGuess{h->gs, h->pp_prev, h->prm.initial_guess == MC_GUESS_LEARNED ? h->x0_learned : nullptr,
+                                h->pv.r, h->pv.q};
+                x2 = h->ir_x2;
+                ir_init(h->stream, A, v.b, v.x, nullptr, h->r32, v.st, v.partials, v.counter, h->prm.p_rtol, 0.0,
+                        IR_MAX_OUTER, 0, g);
+                ok = capture_loop(h, 0, &v.st->done, [&] {
+                    pcg_init_amg<float>(h->stream, A32, in, h->prm.ir_inner_rtol, 0.0, h->prm.max_iters, 0, 0, v.st);
+                    amg_vcycle<float>(h->stream, h->amg, in.r, in.zp[0], in.st, in.partials, in.counter, 1);
+                    const bool inner = capture_loop(h, 1, &in.st->done, [&] {
+                        for (int pin = 0; pin < LOOP_ITERS; pin++) {
+                            pcg_iter1<float>(h->stream, A32, in, pin & 1);
+                            pcg_iter2_amg<float>(h->stream, A32, in, (pin & 1) ^ 1);
+                            amg_vcycle<float>(h->stream, h->amg, in.r, in.zp[(pin & 1) ^ 1], in.st, in.partials,
+                                              in.counter, 0);
+                        }
+                        return true;
+                    });
+                    ir_residual_alt(h->stream, A, v.b, v.x, h->ir_x2, h->r32, v.st, v.partials, v.counter, in.x,
+                                    in.st);
+                    return inner;
+                });
+            } else {
+                pcg_init_amg(h->stream, A, v, h->prm.p_rtol, 0.0, h->prm.max_iters, 1, use_x0);
+                amg_vcycle<double>(h->stream, h->amg, v.r, v.zp[0], v.st, v.partials, v.counter, 1);
+                ok = capture_loop(h, 0, &v.st->done, [&] {
+                    for (int pin = 0; pin < LOOP_ITERS; pin++) {
+                        pcg_iter1(h->stream, A, v, pin & 1);
+                        pcg_iter2_amg(h->stream, A, v, (pin & 1) ^ 1);
+                        amg_vcycle<double>(h->stream, h->amg, v.r, v.zp[(pin & 1) ^ 1], v.st, v.partials, v.counter,
+                                           0);
+                    }
+                    return true;
+                });
+            }
+            pcg_xmean(h->stream, h->N, v, x2);
+            pcg_finish(h->stream, h->N, v, x2, h->pp_prev, h->ph.cell0, h->scalars, h->scalars + 4);
+            launch_corrections(h, 1, 0);
+            ok = cudaMemcpyAsync(h->h_pcg, v.st, sizeof(PcgState), cudaMemcpyDeviceToHost, h->stream) == cudaSuccess && ok;
+            ok = cudaMemcpyAsync(h->h_scalars, h->scalars, 5 * sizeof(double), cudaMemcpyDeviceToHost, h->stream) ==
+                     cudaSuccess && ok;
+            h->launches = before;
+            cudaGraph_t g = nullptr;
+            ok = cudaStreamEndCapture(h->stream, &g) == cudaSuccess && ok;
+            ok = ok && cudaGraphInstantiate(&h->g_corr, g, 0) == cudaSuccess;
+            if (g) cudaGraphDestroy(g);
+        }
+        if (!ok) {
+            cudaGetLastError();
+            h->g_corr = nullptr;
+            h->corr_failed = true;
+            return false;
+        }
+    }
+    if (cudaGraphLaunch(h->g_corr, h->stream) != cudaSuccess) {
+        cudaGetLastError();
+        h->corr_failed = true;
+        return false;
+    }
+    return true;
+}
+
 // Gradients of the six other scalars, with those of u, v, w, p, T at the
 // start of a pass (get_phi_gradients computes all eleven, FlowSolver.inl:917-1063).
 void launch_gradients_scalars(mc_flow *h)
@@ -1230,7 +1393,51 @@ int stage_pressure(mc_flow *h, mc_iter_stats *st)
     if (rc) return rc;
     int loop = 0, worst = MC_OK;
     double pc_ref = 0.0;
-    for (;;) {
+    bool more = true;
+    h->corrector = 1;
+    h->p_bnorm_ref = 0.0;
+    if (use_loops(h) && !h->corr_failed && h->use_amg && simple && !h->snap) {
+        const Ell A = pressure_matrix(h);
+        launch(h, K_PCG_MEAN, [&] { pcg_mean(h->stream, A, h->pv); });
+        const int use_x0 = select_guess(h, A, h->pv.b, h->pv.st, h->pv.x, h->refined);
+        h->guess_used = use_x0 != 0;
+        if ((rc = launch_deferred_inverse(h))) return rc;
+        if (corrector_graph(h, use_x0)) {
+            loop = 1;
+            CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+            if ((rc = check_launch(h))) return rc;
+            if ((rc = check_guess(h))) return rc;
+            const PcgState &ps = *h->h_pcg;
+            const int its = h->refined ? ps.inner_total : ps.iter;
+            const int per_iter = 2 + amg_kernels_per_vcycle(h->amg, h->refined);
+            h->launches += 6 + loop_launches(its, per_iter) + (h->refined ? ps.iter * (per_iter + 1) : per_iter);
+            worst = krylov_status_to_mc(ps.status);
+            h->p_bnorm_ref = std::sqrt(ps.bb);
+            pc_ref = h->h_scalars[0];
+            if (st) {
+                const double relres = ps.bb > 0 ? std::sqrt(ps.rr / ps.bb) : 0.0;
+                st->pressure_solves++;
+                st->pressure_iters_total += its;
+                st->pressure_iters_first = its;
+                st->guess_choice_first = h->guess_choice;
+                st->guess_rel_residual_first = h->guess_rel;
+                st->pressure_rel_residual_first = relres;
+                st->pressure_rel_residual = std::max(st->pressure_rel_residual, relres);
+                st->pressure_correction_max_first = pc_ref;
+            }
+            if (!std::isfinite(pc_ref)) return fail(h, MC_ERR_NONFINITE, "pressure correction is not finite");
+            more = pc_ref > 0.25 * pc_ref;
+            // A zero right-hand side (orthogonal faces: no flux correction)
+            // solves to zero: the second corrector would only leave the
+            // previous correction zero.
+            if (more && h->h_scalars[4] == 0.0) {
+                if (st) st->pressure_solves++;
+                CUDA_TRY(h, cudaMemsetAsync(h->pp_prev, 0, (size_t)h->N * sizeof(double), h->stream));
+                more = false;
+            }
+        }
+    }
+    while (more) {
         loop++;
         int its = 0;
         double relres = 0.0, bnorm = 0.0;
@@ -1273,25 +1480,8 @@ int stage_pressure(mc_flow *h, mc_iter_stats *st)
                                                                        h->scalars);
         });
         CUDA_TRY(h, cudaMemcpyAsync(h->h_scalars, h->scalars, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-        launch_gradient_pressure(h, G_PP);
-        CorrectArgs c{};
-        c.PP = h->phi[G_PP];
-        c.P = h->phi[G_P];
-        c.U = h->phi[G_U];
-        c.V = h->phi[G_V];
-        c.W = h->phi[G_W];
-        c.AU = h->AU;
-        for (int d = 0; d < 3; d++) c.gPP[d] = h->grad[G_PP][d];
-        c.ff0 = h->ff0;
-        c.mdot = h->mdot;
-        c.fcorr = h->fcorr;
-        c.next_rhs = simple ? h->b_p : nullptr;
-        const int grid_f = std::min(blocks_for(h->F), krylov_grid(h->F));
-        launch(h, K_PP_FACES, [&] { k_pp_correct_faces<<<grid_f, MCB_THREADS, 0, h->stream>>>(h->ph, h->margs, c); });
         const int cell0 = (!simple && h->first_pressure) ? 1 : 0;
-        launch(h, K_PP_CELLS, [&] {
-            k_pp_correct_cells<<<blocks_for(h->N + 6), MCB_THREADS, 0, h->stream>>>(h->ph, h->margs, c, simple, cell0);
-        });
+        launch_corrections(h, simple, cell0);
         if (cell0) h->first_pressure = 0;
         CUDA_TRY(h, cudaStreamSynchronize(h->stream));
         flush_timing(h);
@@ -2308,7 +2498,7 @@ int mc_flow_destroy(mc_flow *h)
     if (h->scal_mem) cudaFree(h->scal_mem);
     if (h->node_mem) cudaFree(h->node_mem);
     if (h->xin_mem) cudaFree(h->xin_mem);
-    for (cudaGraphExec_t g : {h->g_bs, h->l_bs})
+    for (cudaGraphExec_t g : {h->g_bs, h->l_bs, h->g_corr})
         if (g) cudaGraphExecDestroy(g);
     for (void *p : {(void *)h->h_bi3, (void *)h->h_bi1, (void *)h->h_bo3, (void *)h->h_bo1, (void *)h->h_sweep3,
                     (void *)h->h_sweep1})
@@ -2316,6 +2506,8 @@ int mc_flow_destroy(mc_flow *h)
     if (h->side) cudaStreamSynchronize(h->side);  // no inverse still being formed into freed memory
     if (h->stream) cudaStreamDestroy(h->stream);
     if (h->side) cudaStreamDestroy(h->side);
+    for (cudaStream_t c : h->cap)
+        if (c) cudaStreamDestroy(c);
     if (h->ev_levels) cudaEventDestroy(h->ev_levels);
     if (h->ev_inverse) cudaEventDestroy(h->ev_inverse);
     delete h;

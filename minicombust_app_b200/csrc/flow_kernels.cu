@@ -1075,6 +1075,7 @@ __global__ void __launch_bounds__(MCB_THREADS, 4) k_pp_correct_cells(Physics ph,
 {
     const int N = ph.N;
     const int c = grid_stride_start();
+    double rmax = 0.0;
     if (c < N) {
         if (correct_all || (correct_cell0 && c == ph.cell0)) {
             const double A = a.AU[c];
@@ -1098,11 +1099,15 @@ __global__ void __launch_bounds__(MCB_THREADS, 4) k_pp_correct_cells(Physics ph,
                     s += a.fcorr[face];
             }
             a.next_rhs[c] = s;
+            rmax = isnan(s) ? 1.0 / 0.0 : fabs(s);
         }
         a.PP[c] = 0.0;
     } else if (c < N + 6) {
         a.PP[c] = 0.0;
     }
+    // (no atomics where it is zero everywhere: orthogonal meshes)
+    if (a.rhs_max && rmax > 0.0)
+        atomicMax((unsigned long long *)a.rhs_max, (unsigned long long)__double_as_longlong(rmax));
 }
 
 // update_P (FlowSolver.inl:2292-2315): boundary pressure from the last face

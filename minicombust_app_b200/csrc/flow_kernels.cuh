@@ -132,6 +132,7 @@ struct CorrectArgs {
     const double *ff0;
     double *mdot, *fcorr;
     double *next_rhs;           // null: do not build the next corrector's right-hand side
+    double *rhs_max;            // max |next_rhs| (zero before the launch); null: not formed
 };
 
 // The gradient kernel is a template; it is launched from its own translation

@@ -223,11 +223,12 @@ __global__ void __launch_bounds__(MCB_THREADS) k_pcg_iter2(Ell A, PcgVectors v, 
 template <typename T>
 __global__ void __launch_bounds__(MCB_THREADS) k_pcg_init_amg(EllT<T> A, PcgVectorsT<T> v, double rtol,
                                                               double abs_floor, int max_iters, int project,
-                                                              int use_x0)
+                                                              int use_x0, const PcgState *__restrict__ outer)
 {
     using T2 = typename Pair<T>::type;
     __shared__ double sh[2][MCB_THREADS];
     const int N = A.N;
+    if (outer) rtol = fmin(0.5, fmax(rtol, outer->rr > 0.0 ? 0.5 * sqrt(outer->tol2 / outer->rr) : rtol));
     const double mean = project ? v.st->mean : 0.0;
     double acc[2] = {0.0, 0.0};  // b.b, r.r
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
@@ -383,6 +384,7 @@ __global__ void __launch_bounds__(MCB_THREADS) k_ir_init(Ell A, const double *__
             const double t = fmax(rtol * sqrt(tot[0]), abs_floor);
             st->tol2 = t * t;
             st->iter = 0;
+            st->inner_total = 0;
             st->max_iters = max_outer;
             st->status = KRYLOV_OK;
             st->done = (tot[0] == 0.0 || tot[1] <= st->tol2) ? 1 : 0;
@@ -474,15 +476,19 @@ __global__ void __launch_bounds__(MCB_THREADS) k_guess_apply(int N, double *__re
 // evaluated at each row where the product needs it and stored in xout (not
 // in x, which neighbouring rows still read); without e, x' = x.  r may be
 // null (the FP64 residual is then not stored).
-__global__ void __launch_bounds__(MCB_THREADS) k_ir_residual(Ell A, const double *__restrict__ b,
-                                                             const double *__restrict__ x, const float *__restrict__ e,
-                                                             double *__restrict__ xout, double *__restrict__ r,
-                                                             float *__restrict__ r32, PcgState *st, double *partials,
-                                                             unsigned int *counter)
+// With alt set x and xout change places when st->iter is odd (ir_residual_alt).
+__global__ void __launch_bounds__(MCB_THREADS) k_ir_residual(Ell A, const double *__restrict__ b, const double *x0,
+                                                             const float *__restrict__ e, double *x1,
+                                                             double *__restrict__ r, float *__restrict__ r32,
+                                                             PcgState *st, double *partials, unsigned int *counter,
+                                                             int alt, const PcgState *inner)
 {
     pdl_wait();
     __shared__ double sh[1][MCB_THREADS];
     const int N = A.N;
+    const bool odd = alt && (st->iter & 1);
+    const double *__restrict__ x = odd ? x1 : x0;
+    double *__restrict__ xout = odd ? const_cast<double *>(x0) : x1;
     if (st->done) {  // nothing to add: xout still has to hold the solution
         if (e)
             for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) xout[i] = x[i];
@@ -511,6 +517,7 @@ __global__ void __launch_bounds__(MCB_THREADS) k_ir_residual(Ell A, const double
         if (threadIdx.x == 0) {
             st->rr = tot[0];
             st->iter += 1;
+            if (inner) st->inner_total += inner->iter;
             if (!finite(tot[0])) {
                 st->done = 1;
                 st->status = KRYLOV_NONFINITE;
@@ -524,11 +531,12 @@ __global__ void __launch_bounds__(MCB_THREADS) k_ir_residual(Ell A, const double
     }
 }
 
-__global__ void __launch_bounds__(MCB_THREADS) k_pcg_xmean(int N, PcgVectors v)
+__global__ void __launch_bounds__(MCB_THREADS) k_pcg_xmean(int N, PcgVectors v, const double *x2)
 {
     __shared__ double sh[1][MCB_THREADS];
+    const double *__restrict__ x = (x2 && (v.st->iter & 1)) ? x2 : v.x;
     double acc[1] = {0.0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) acc[0] += v.x[i];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) acc[0] += x[i];
     if (publish_partials<1>(acc, v.partials, v.counter, sh)) {
         double tot[1];
         reduce_partials<1>(tot, v.partials, v.counter, sh);
@@ -540,6 +548,30 @@ __global__ void __launch_bounds__(MCB_THREADS) k_pcg_sub_xmean(int N, PcgVectors
 {
     const double m = v.st->xmean;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) v.x[i] -= m;
+}
+
+__global__ void __launch_bounds__(MCB_THREADS) k_pcg_finish(int N, PcgVectors v, const double *x2,
+                                                            double *__restrict__ prev, int cell0, double *pp_max,
+                                                            double *zero)
+{
+    __shared__ double sh[1][MCB_THREADS];
+    const double m = v.st->xmean;
+    const double *x = (x2 && (v.st->iter & 1)) ? x2 : v.x;
+    double acc[1] = {-1.0e308};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+        const double xi = x[i] - m;
+        v.x[i] = xi;
+        prev[i] = xi;
+        acc[0] = fmax(acc[0], i == cell0 ? xi : fabs(xi));
+    }
+    if (publish_partials<1, true>(acc, v.partials, v.counter, sh)) {
+        double tot[1];
+        reduce_partials<1, true>(tot, v.partials, v.counter, sh);
+        if (threadIdx.x == 0) {
+            *pp_max = tot[0];
+            *zero = 0.0;
+        }
+    }
 }
 
 void pcg_mean(cudaStream_t s, const Ell &A, const PcgVectors &v)
@@ -562,9 +594,10 @@ void pcg_iter2(cudaStream_t s, const Ell &A, const PcgVectors &v, int pnew)
 }
 template <typename T>
 void pcg_init_amg(cudaStream_t s, const EllT<T> &A, const PcgVectorsT<T> &v, double rtol, double abs_floor,
-                  int max_iters, int project, int use_x0)
+                  int max_iters, int project, int use_x0, const PcgState *outer)
 {
-    k_pcg_init_amg<T><<<krylov_grid(A.N), MCB_THREADS, 0, s>>>(A, v, rtol, abs_floor, max_iters, project, use_x0);
+    k_pcg_init_amg<T><<<krylov_grid(A.N), MCB_THREADS, 0, s>>>(A, v, rtol, abs_floor, max_iters, project, use_x0,
+                                                               outer);
 }
 template <typename T>
 void pcg_iter2_amg(cudaStream_t s, const EllT<T> &A, const PcgVectorsT<T> &v, int pnew)
@@ -574,7 +607,7 @@ void pcg_iter2_amg(cudaStream_t s, const EllT<T> &A, const PcgVectorsT<T> &v, in
 #define MCB_INSTANTIATE_PCG(T)                                                                                  \
     template void pcg_iter1<T>(cudaStream_t, const EllT<T> &, const PcgVectorsT<T> &, int);                   \
     template void pcg_init_amg<T>(cudaStream_t, const EllT<T> &, const PcgVectorsT<T> &, double, double, int, \
-                                  int, int);                                                                  \
+                                  int, int, const PcgState *);                                                                  \
     template void pcg_iter2_amg<T>(cudaStream_t, const EllT<T> &, const PcgVectorsT<T> &, int);
 MCB_INSTANTIATE_PCG(double)
 MCB_INSTANTIATE_PCG(float)
@@ -598,9 +631,24 @@ void guess_apply(cudaStream_t s, int N, double *x, const double *xa, const doubl
 void ir_residual(cudaStream_t s, const Ell &A, const double *b, const double *x, double *r, float *r32, PcgState *st,
                  double *partials, unsigned int *counter, const float *e, double *xout)
 {
-    k_ir_residual<<<krylov_grid(A.N), MCB_THREADS, 0, s>>>(A, b, x, e, xout, r, r32, st, partials, counter);
+    k_ir_residual<<<krylov_grid(A.N), MCB_THREADS, 0, s>>>(A, b, x, e, xout, r, r32, st, partials, counter, 0,
+                                                          nullptr);
 }
-void pcg_xmean(cudaStream_t s, int N, const PcgVectors &v) { k_pcg_xmean<<<krylov_grid(N), MCB_THREADS, 0, s>>>(N, v); }
+void ir_residual_alt(cudaStream_t s, const Ell &A, const double *b, double *x, double *x2, float *r32, PcgState *st,
+                     double *partials, unsigned int *counter, const float *e, const PcgState *inner)
+{
+    k_ir_residual<<<krylov_grid(A.N), MCB_THREADS, 0, s>>>(A, b, x, e, x2, nullptr, r32, st, partials, counter, 1,
+                                                          inner);
+}
+void pcg_xmean(cudaStream_t s, int N, const PcgVectors &v, const double *x2)
+{
+    k_pcg_xmean<<<krylov_grid(N), MCB_THREADS, 0, s>>>(N, v, x2);
+}
+void pcg_finish(cudaStream_t s, int N, const PcgVectors &v, const double *x2, double *prev, int cell0, double *pp_max,
+                double *zero)
+{
+    k_pcg_finish<<<krylov_grid(N), MCB_THREADS, 0, s>>>(N, v, x2, prev, cell0, pp_max, zero);
+}
 void pcg_sub_xmean(cudaStream_t s, int N, const PcgVectors &v)
 {
     k_pcg_sub_xmean<<<krylov_grid(N), MCB_THREADS, 0, s>>>(N, v);

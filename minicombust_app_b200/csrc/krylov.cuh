@@ -208,6 +208,7 @@ __device__ __forceinline__ void row_cols(const EllT<T> &A, int i, int (&c)[6])
 struct PcgState {
     double rz, rz_old, alpha, pq, rr, bb, tol2, mean, xmean;
     int iter, done, status, max_iters;
+    int inner_total;  // refinement: iterations of the inner solves so far
 };
 
 template <int R>
@@ -347,9 +348,12 @@ void pcg_iter1(cudaStream_t s, const EllT<T> &A, const PcgVectorsT<T> &v, int pi
 void pcg_iter2(cudaStream_t s, const Ell &A, const PcgVectors &v, int pnew);
 // AMG-preconditioned variant: init without z, update without z (amg.cu
 // computes z and r . z after each update).
+// With outer given (the state of the refinement around an inner solve) rtol is
+// the smallest tolerance to ask for, and the one asked for is formed here:
+// the reduction outer still misses, with a margin of 2, and at most 0.5.
 template <typename T>
 void pcg_init_amg(cudaStream_t s, const EllT<T> &A, const PcgVectorsT<T> &v, double rtol, double abs_floor,
-                  int max_iters, int project, int use_x0 = 0);
+                  int max_iters, int project, int use_x0 = 0, const PcgState *outer = nullptr);
 template <typename T>
 void pcg_iter2_amg(cudaStream_t s, const EllT<T> &A, const PcgVectorsT<T> &v, int pnew);
 // FP64 iterative refinement around an FP32 inner solve: the state's mean
@@ -386,8 +390,17 @@ void guess_residuals(cudaStream_t s, const Ell &A, const double *b, const PcgSta
 void guess_apply(cudaStream_t s, int N, double *x, const double *xa, const double *xb, const GuessState *gs);
 void ir_residual(cudaStream_t s, const Ell &A, const double *b, const double *x, double *r, float *r32, PcgState *st,
                  double *partials, unsigned int *counter, const float *e = nullptr, double *xout = nullptr);
-void pcg_xmean(cudaStream_t s, int N, const PcgVectors &v);
+// The same inside a device loop: the solution alternates between x and x2 by
+// the parity of st->iter (x first), and inner's iterations are added up.
+void ir_residual_alt(cudaStream_t s, const Ell &A, const double *b, double *x, double *x2, float *r32, PcgState *st,
+                     double *partials, unsigned int *counter, const float *e, const PcgState *inner);
+// x2 (may be null): the solution is there when st->iter is odd.
+void pcg_xmean(cudaStream_t s, int N, const PcgVectors &v, const double *x2 = nullptr);
 void pcg_sub_xmean(cudaStream_t s, int N, const PcgVectors &v);
+// v.x = solution - mean, its copy in prev, and the largest correction (as
+// k_pp_max) in *pp_max; *zero = 0 for the kernel that follows.
+void pcg_finish(cudaStream_t s, int N, const PcgVectors &v, const double *x2, double *prev, int cell0, double *pp_max,
+                double *zero);
 
 template <typename T, int R>
 void bicg_init_t(cudaStream_t s, const EllT<T> &A, const BicgVectorsT<T, R> &v, double rtol, int max_iters);
