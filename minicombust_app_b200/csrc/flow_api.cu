@@ -208,6 +208,7 @@ struct mc_flow {
 
     // the other scalar transports (transport_scalars): TE, ED, TP, FUL, PRO,
     // VARF, VARP fields and the gradients of all but TP, by MC_FIELD id
+    bool ortho = false;  // every internal face's cell centres lie on its normal line (launch_face_offsets)
     bool has_scalars = false;
     char *scal_mem = nullptr;
     double *sfield[MC_FIELD_VARP + 1] = {};
@@ -1112,10 +1113,9 @@ void launch_corrections(mc_flow *h, int simple, int cell0)
     c.next_rhs = simple ? h->b_p : nullptr;
     c.rhs_max = simple ? h->scalars + 4 : nullptr;
     const int grid_f = std::min(blocks_for(h->F), krylov_grid(h->F));
-    launch(h, K_PP_FACES, [&] { k_pp_correct_faces<<<grid_f, MCB_THREADS, 0, h->stream>>>(h->ph, h->margs, c); });
-    launch(h, K_PP_CELLS, [&] {
-        k_pp_correct_cells<<<blocks_for(h->N + 6), MCB_THREADS, 0, h->stream>>>(h->ph, h->margs, c, simple, cell0);
-    });
+    launch(h, K_PP_FACES, [&] { launch_pp_correct_faces(h->stream, grid_f, h->ortho, h->ph, h->margs, c); });
+    launch(h, K_PP_CELLS,
+           [&] { launch_pp_correct_cells(h->stream, h->ortho, h->ph, h->margs, c, simple, cell0); });
 }
 
 // The first corrector of a simple-mode pass with AMG, from the solve's
@@ -2461,6 +2461,14 @@ int mc_flow_create(const mc_mesh_view *mesh, const mc_flow_params *params, mc_fl
             m.xc = h->xc; m.yc = h->yc; m.zc = h->zc;
             m.vol = h->vol; m.rho = h->rho;
             m.outlet_faces = h->outlet_faces;
+            // (the boundary balance's memory takes the flag: nothing has run yet)
+            int *flag = reinterpret_cast<int *>(h->balance), off = 1;
+            launch_face_offsets(h->stream, krylov_grid(h->F), h->N, m, flag);
+            if (cudaMemcpyAsync(&off, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
+                cudaStreamSynchronize(h->stream) != cudaSuccess)
+                rc = fail(h, MC_ERR_CUDA, "face offsets");
+            h->ortho = off == 0;
+            cudaMemsetAsync(h->balance, 0, sizeof(FluxBalance), h->stream);
         }
     }
     if (!rc) {

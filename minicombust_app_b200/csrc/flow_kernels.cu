@@ -38,6 +38,26 @@ __device__ __forceinline__ void cramer(double A00, double A10, double A20, doubl
          (b2 * invdet * (A00 * A11 - A10 * A01));
 }
 
+// S / |S| with |S| = sqrt(S . S).  Where two components are zero (axis-aligned
+// faces) sqrt(s * s) = |s| exactly and the quotients are +-1 and 0, the same
+// values without the square root and the three divisions, whose chain is a
+// third of the flux kernel's FP64 work; squares neither over- nor underflow
+// inside the bounds.
+__device__ __forceinline__ void unit_normal(double Sx, double Sy, double Sz, double &nx, double &ny, double &nz)
+{
+    const double s = Sx + Sy + Sz, a = fabs(s);
+    if ((Sx != 0.0) + (Sy != 0.0) + (Sz != 0.0) == 1 && a > 1e-140 && a < 1e140) {
+        nx = Sx != 0.0 ? copysign(1.0, Sx) : 0.0;
+        ny = Sy != 0.0 ? copysign(1.0, Sy) : 0.0;
+        nz = Sz != 0.0 ? copysign(1.0, Sz) : 0.0;
+        return;
+    }
+    const double smag = sqrt(Sx * Sx + Sy * Sy + Sz * Sz);
+    nx = Sx / smag;
+    ny = Sy / smag;
+    nz = Sz / smag;
+}
+
 __device__ __forceinline__ int grid_stride_start() { return blockIdx.x * blockDim.x + threadIdx.x; }
 
 // The FP32 copy of an assembled row for the refined solves, written by the
@@ -866,8 +886,8 @@ __global__ void __launch_bounds__(MCB_THREADS, 4) k_mass_flux(Physics ph, MeshAr
             const double WF = a.W[c1] * l1 + a.W[c0] * l0 + (dWx * dlx + dWy * dly + dWz * dlz);
             const double densityf = m.rho[c0] * l0 + m.rho[c1] * l1;
             double md = densityf * (UF * Sx + VF * Sy + WF * Sz);
-            const double smag = sqrt(Sx * Sx + Sy * Sy + Sz * Sz);
-            const double nx = Sx / smag, ny = Sy / smag, nz = Sz / smag;
+            double nx, ny, nz;
+            unit_normal(Sx, Sy, Sz, nx, ny, nz);
             const double d0 = (xf - x0) * nx + (yf - y0) * ny + (zf - z0) * nz;
             const double d1 = (xf - x1) * nx + (yf - y1) * ny + (zf - z1) * nz;
             const double Xpacx = xf - nx * d0, Xpacy = yf - ny * d0, Xpacz = zf - nz * d0;
@@ -1029,8 +1049,53 @@ __global__ void __launch_bounds__(MCB_THREADS) k_dir_rows64(int N, const double 
 }
 
 // ------------------------------------------------------- corrector updates
+// The projections of a face's two cell centres onto the face's normal line,
+// less the centres, with rounding below 3e-16 taken as zero (update_mass_flux,
+// FlowSolver.inl:1812-1878): what the non-orthogonal flux correction multiplies
+// the correction's gradients with.
+__device__ __forceinline__ void face_offsets(const MeshArgs &m, int face, int c0, int c1, double (&Xn)[3],
+                                             double (&Xp)[3])
+{
+    double nx, ny, nz;
+    unit_normal(m.Sx[face], m.Sy[face], m.Sz[face], nx, ny, nz);
+    const double x0 = m.xc[c0], y0 = m.yc[c0], z0 = m.zc[c0];
+    const double x1 = m.xc[c1], y1 = m.yc[c1], z1 = m.zc[c1];
+    const double xf = m.xf[face], yf = m.yf[face], zf = m.zf[face];
+    const double d0 = (xf - x0) * nx + (yf - y0) * ny + (zf - z0) * nz;
+    const double d1 = (xf - x1) * nx + (yf - y1) * ny + (zf - z1) * nz;
+    Xn[0] = (xf - nx * d1) - x1;
+    Xn[1] = (yf - ny * d1) - y1;
+    Xn[2] = (zf - nz * d1) - z1;
+    Xp[0] = (xf - nx * d0) - x0;
+    Xp[1] = (yf - ny * d0) - y0;
+    Xp[2] = (zf - nz * d0) - z0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        if (fabs(Xn[d]) < 0.0000000000000003) Xn[d] = 0.0;
+        if (fabs(Xp[d]) < 0.0000000000000003) Xp[d] = 0.0;
+    }
+}
+
+// Whether some internal face has a non-zero offset: *flag = 1.
+__global__ void __launch_bounds__(MCB_THREADS) k_face_offsets(int N, MeshArgs m, int *flag)
+{
+    for (int face = grid_stride_start(); face < m.F; face += gridDim.x * blockDim.x) {
+        const int c0 = m.fc0[face], c1 = m.fc1[face];
+        if (c1 >= N) continue;
+        double Xn[3], Xp[3];
+        face_offsets(m, face, c0, c1, Xn, Xp);
+        if (Xn[0] != 0.0 || Xn[1] != 0.0 || Xn[2] != 0.0 || Xp[0] != 0.0 || Xp[1] != 0.0 || Xp[2] != 0.0) *flag = 1;
+    }
+}
+
 // Face part of one corrector pass of calculate_pressure: mass flux += a_f
 // (PP_N - PP_P) (:2402-2412) then update_mass_flux (:1812-1878).
+// ORTHO: no internal face has an offset (k_face_offsets at creation), so the
+// flux correction is zero and neither it nor what it is formed from -- normals,
+// centres, gradients: three quarters of the kernel's bytes -- is touched
+// (timestep of the plain 2 x 128^3 box 25.7 -> 24.8 ms with the cells' part and
+// the flux kernel's unit_normal).
+template <bool ORTHO>
 __global__ void __launch_bounds__(MCB_THREADS, 4) k_pp_correct_faces(Physics ph, MeshArgs m, CorrectArgs a)
 {
     const int N = ph.N, F = m.F;
@@ -1040,36 +1105,25 @@ __global__ void __launch_bounds__(MCB_THREADS, 4) k_pp_correct_faces(Physics ph,
         const double fact = a.ff0[face];
         double md = a.mdot[face];
         md += (fact * (a.PP[c1] - a.PP[c0]));
-        const double Sx = m.Sx[face], Sy = m.Sy[face], Sz = m.Sz[face];
-        const double smag = sqrt(Sx * Sx + Sy * Sy + Sz * Sz);
-        const double nx = Sx / smag, ny = Sy / smag, nz = Sz / smag;
-        const double x0 = m.xc[c0], y0 = m.yc[c0], z0 = m.zc[c0];
-        const double x1 = m.xc[c1], y1 = m.yc[c1], z1 = m.zc[c1];
-        const double xf = m.xf[face], yf = m.yf[face], zf = m.zf[face];
-        const double d0 = (xf - x0) * nx + (yf - y0) * ny + (zf - z0) * nz;
-        const double d1 = (xf - x1) * nx + (yf - y1) * ny + (zf - z1) * nz;
-        double Xnx = (xf - nx * d1) - x1, Xny = (yf - ny * d1) - y1, Xnz = (zf - nz * d1) - z1;
-        double Xpx = (xf - nx * d0) - x0, Xpy = (yf - ny * d0) - y0, Xpz = (zf - nz * d0) - z0;
-        if (fabs(Xnx) < 0.0000000000000003) Xnx = 0.0;
-        if (fabs(Xny) < 0.0000000000000003) Xny = 0.0;
-        if (fabs(Xnz) < 0.0000000000000003) Xnz = 0.0;
-        if (fabs(Xpx) < 0.0000000000000003) Xpx = 0.0;
-        if (fabs(Xpy) < 0.0000000000000003) Xpy = 0.0;
-        if (fabs(Xpz) < 0.0000000000000003) Xpz = 0.0;
-        const double dpx = a.gPP[0][c1] * Xnx - a.gPP[0][c0] * Xpx;
-        const double dpy = a.gPP[1][c1] * Xny - a.gPP[1][c0] * Xpy;
-        const double dpz = a.gPP[2][c1] * Xnz - a.gPP[2][c0] * Xpz;
-        const double fc = fact * (dpx + dpy + dpz) * ph.flux_corr;
-        md += fc;
+        if (!ORTHO) {
+            double Xn[3], Xp[3];
+            face_offsets(m, face, c0, c1, Xn, Xp);
+            const double dpx = a.gPP[0][c1] * Xn[0] - a.gPP[0][c0] * Xp[0];
+            const double dpy = a.gPP[1][c1] * Xn[1] - a.gPP[1][c0] * Xp[1];
+            const double dpz = a.gPP[2][c1] * Xn[2] - a.gPP[2][c0] * Xp[2];
+            const double fc = fact * (dpx + dpy + dpz) * ph.flux_corr;
+            md += fc;
+            a.fcorr[face] = fc;
+        }
         a.mdot[face] = md;
-        a.fcorr[face] = fc;
     }
 }
 
 // Cell part: P += urf_p PP and u -= V/A grad(PP) (:2416-2433; every cell in
 // simple mode, only cell 0 on the first call in compat mode), the next
 // corrector's right-hand side from the non-orthogonal flux corrections
-// (:1875-1876, simple mode), and PP = 0 (:2447-2450).
+// (:1875-1876, simple mode; zero with ORTHO), and PP = 0 (:2447-2450).
+template <bool ORTHO>
 __global__ void __launch_bounds__(MCB_THREADS, 4) k_pp_correct_cells(Physics ph, MeshArgs m, CorrectArgs a,
                                                                   int correct_all, int correct_cell0)
 {
@@ -1088,26 +1142,47 @@ __global__ void __launch_bounds__(MCB_THREADS, 4) k_pp_correct_cells(Physics ph,
         }
         if (a.next_rhs) {
             double s = 0.0;
+            if (!ORTHO) {
 #pragma unroll
-            for (int k = 0; k < 6; k++) {
-                const int face = m.sface[(size_t)k * N + c];
-                const int c0 = m.fc0[face], c1 = m.fc1[face];
-                if (c1 >= N) continue;
-                if (c == c0)
-                    s -= a.fcorr[face];
-                else
-                    s += a.fcorr[face];
+                for (int k = 0; k < 6; k++) {
+                    const int face = m.sface[(size_t)k * N + c];
+                    const int c0 = m.fc0[face], c1 = m.fc1[face];
+                    if (c1 >= N) continue;
+                    if (c == c0)
+                        s -= a.fcorr[face];
+                    else
+                        s += a.fcorr[face];
+                }
+                rmax = isnan(s) ? 1.0 / 0.0 : fabs(s);
             }
             a.next_rhs[c] = s;
-            rmax = isnan(s) ? 1.0 / 0.0 : fabs(s);
         }
         a.PP[c] = 0.0;
     } else if (c < N + 6) {
         a.PP[c] = 0.0;
     }
-    // (no atomics where it is zero everywhere: orthogonal meshes)
-    if (a.rhs_max && rmax > 0.0)
+    // (no atomics where it is zero everywhere)
+    if (!ORTHO && a.rhs_max && rmax > 0.0)
         atomicMax((unsigned long long *)a.rhs_max, (unsigned long long)__double_as_longlong(rmax));
+}
+
+void launch_face_offsets(cudaStream_t s, int grid, int N, const MeshArgs &m, int *flag)
+{
+    k_face_offsets<<<grid, MCB_THREADS, 0, s>>>(N, m, flag);
+}
+
+void launch_pp_correct_faces(cudaStream_t s, int grid, bool ortho, const Physics &ph, const MeshArgs &m,
+                             const CorrectArgs &a)
+{
+    (ortho ? k_pp_correct_faces<true> : k_pp_correct_faces<false>)<<<grid, MCB_THREADS, 0, s>>>(ph, m, a);
+}
+
+void launch_pp_correct_cells(cudaStream_t s, bool ortho, const Physics &ph, const MeshArgs &m, const CorrectArgs &a,
+                             int correct_all, int correct_cell0)
+{
+    const int grid = (ph.N + 6 + MCB_THREADS - 1) / MCB_THREADS;
+    (ortho ? k_pp_correct_cells<true> : k_pp_correct_cells<false>)<<<grid, MCB_THREADS, 0, s>>>(
+        ph, m, a, correct_all, correct_cell0);
 }
 
 // update_P (FlowSolver.inl:2292-2315): boundary pressure from the last face

@@ -162,8 +162,13 @@ __global__ void k_mass_flux(Physics ph, MeshArgs m, MassFluxArgs a);
 __global__ void k_outlet_fix(Physics ph, MeshArgs m, double *mdot, double *U, double *V, double *W,
                              const FluxBalance *bal);
 __global__ void k_pressure_rows(Physics ph, MeshArgs m, PressureRowArgs a);
-__global__ void k_pp_correct_faces(Physics ph, MeshArgs m, CorrectArgs a);
-__global__ void k_pp_correct_cells(Physics ph, MeshArgs m, CorrectArgs a, int correct_all, int correct_cell0);
+// *flag = 1 when the centres of some internal face's cells are off its normal
+// line (zero before the launch); ortho: none are.
+void launch_face_offsets(cudaStream_t s, int grid, int N, const MeshArgs &m, int *flag);
+void launch_pp_correct_faces(cudaStream_t s, int grid, bool ortho, const Physics &ph, const MeshArgs &m,
+                             const CorrectArgs &a);
+void launch_pp_correct_cells(cudaStream_t s, bool ortho, const Physics &ph, const MeshArgs &m, const CorrectArgs &a,
+                             int correct_all, int correct_cell0);
 __global__ void k_update_p_boundary(Physics ph, MeshArgs m, double *P, double *gPx, double *gPy, double *gPz,
                                     const int *nbr);
 __global__ void k_pp_max(int N, int cell0, const double *PP, double *partials, unsigned int *counter, double *out);
