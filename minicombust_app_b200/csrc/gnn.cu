@@ -92,6 +92,20 @@ __device__ __forceinline__ void ldm_x4(uint32_t (&r)[4], const bf16 *p)
                  : "r"(a));
 }
 
+// The same matrices transposed: row addresses run along the reduction dimension.
+__device__ __forceinline__ void ldm_x4_t(uint32_t (&r)[4], const bf16 *p)
+{
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a));
+}
+__device__ __forceinline__ void ldm_x2_t(uint32_t (&r)[2], const bf16 *p)
+{
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(a));
+}
+
 // acc (16 rows x 32 columns) += A[16][16 KS] . W[32][16 KS]^T for one warp,
 // A and W row-major BF16 in shared memory (row strides multiples of 8).
 template <int KS>
@@ -291,23 +305,6 @@ __global__ void __launch_bounds__(GNN_TILE) k_gnn_encode(GnnGraph g, const __gri
         }
         *reinterpret_cast<uint4 *>(hout + (size_t)i * GNN_H + c4 * 8) = o.u;
     }
-}
-
-// Gather of one cell's message for channel `lane` (h is [n][H] BF16).
-struct SlotCache {
-    int col[6];
-    uint32_t edge[6];
-};
-
-__device__ __forceinline__ SlotCache load_slots(const GnnGraph &g, int i)
-{
-    SlotCache s;
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        s.col[k] = i < g.n ? g.col[(size_t)k * g.n + i] : -1;
-        s.edge[k] = i < g.n ? *reinterpret_cast<const uint32_t *>(g.edge + (size_t)k * g.n + i) : 0u;
-    }
-    return s;
 }
 
 __device__ __forceinline__ float2 edge_of(uint32_t bits)
@@ -816,10 +813,9 @@ __global__ void __launch_bounds__(MCB_THREADS) k_gnn_loss_grad(int n, const floa
 // Backward kernels: a block loops over tiles (of all samples of the launch)
 // and keeps its parameter gradients -- the products' accumulators and the
 // channel sums -- in registers, so a launch writes one partial per block
-// (at most BWD_BLOCKS) instead of one per tile.  Rows are read four at a time:
-// the loads of four rows are in flight together (bound by their latency
-// otherwise).  With several samples per launch, a batch of 8 on 65,536 cells
-// takes 4.13 ms where one launch per sample and tile took 5.84 ms.
+// (at most BWD_BLOCKS) instead of one per tile.  Several rows' loads are in
+// flight together (bound by their latency otherwise).  With several samples per launch, a batch of 8 on 65,536 cells
+// takes 1.98 ms where one launch per sample and tile took 5.84 ms.
 struct TileLoop {
     int ntiles, total;  // tiles of a sample, tiles of the launch
 };
@@ -906,149 +902,219 @@ __global__ void __launch_bounds__(GNN_TILE) k_gnn_decode_bwd(GnnGraph g, TileLoo
     if (warp == 0 && lane == 0) gp[GPD_CO] = t_dco;
 }
 
+// Four consecutive channels of a row: an eighth of a warp reads a row.
+union Chunk4 {
+    uint2 u;
+    bf162 h[2];
+};
+__device__ __forceinline__ float4 load_h4(const bf16 *p)
+{
+    Chunk4 v;
+    v.u = *reinterpret_cast<const uint2 *>(p);
+    const float2 a = __bfloat1622float2(v.h[0]), b = __bfloat1622float2(v.h[1]);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void store_h4(bf16 *p, float a, float b, float c, float d)
+{
+    Chunk4 v;
+    v.h[0] = __floats2bfloat162_rn(a, b);
+    v.h[1] = __floats2bfloat162_rn(c, d);
+    *reinterpret_cast<uint2 *>(p) = v.u;
+}
+
+// Slot k of row i: the neighbour (the row itself without one) and the gate of
+// channels c .. c + 3.
+struct Slot4 {
+    int j;
+    float2 e;
+    float g[4];
+};
+__device__ __forceinline__ Slot4 load_slot4(const GnnGraph &g, int k, int i, const float (&wg0)[4],
+                                            const float (&wg1)[4], const float (&cg)[4])
+{
+    Slot4 s;
+    s.j = g.col[(size_t)k * g.n + i];
+    s.e = edge_of(*reinterpret_cast<const uint32_t *>(g.edge + (size_t)k * g.n + i));
+#pragma unroll
+    for (int q = 0; q < 4; q++) s.g[q] = wg0[q] * s.e.x + wg1[q] * s.e.y + cg[q];
+    return s;
+}
+
+// Sum of a per-lane channel quadruple (channels 4 (lane % 8) ..) over the
+// block's rows, warps in order; in warp 0, lane = channel.  red: [8][32].
+__device__ __forceinline__ float block_quad_sum(const float (&v)[4], float (*red)[GNN_H], int warp, int lane)
+{
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        float t = v[q];
+        t += __shfl_xor_sync(FULL, t, 8);
+        t += __shfl_xor_sync(FULL, t, 16);
+        if (lane < 8) red[warp][4 * lane + q] = t;
+    }
+    __syncthreads();
+    float s = 0.f;
+    if (warp == 0) {
+#pragma unroll
+        for (int w = 0; w < 8; w++) s += red[w][lane];
+    }
+    return s;
+}
+
+constexpr int BWD_THREADS = 256;  // 8 warps of 16 rows
+constexpr int LDU = 2 * GNN_H + 8;
+
 // Layer backward, dense part.  In: dho = dL/dh' (FP32), the layer input h and
 // the saved activation a.  Out: dhs = dL/dh through the residual and the
 // self half of u; dm = dL/dm; partial gradients of W1, c1, W2, c2.
-constexpr size_t BWD_SMEM = sizeof(bf16) * ((size_t)2 * GNN_H * LDT      // sUT
-                                            + (size_t)GNN_TILE * LDH     // sDH
-                                            + (size_t)GNN_H * LDT        // sDHT
-                                            + (size_t)GNN_H * LDT        // sAT
-                                            + (size_t)GNN_TILE * LDH     // sDZ
-                                            + (size_t)GNN_H * LDT        // sDZT
-                                            + (size_t)GNN_H * LDH        // sW2T
-                                            + (size_t)2 * GNN_H * LDH)   // sW1T
-                            + sizeof(float) * 4 * GNN_H;
+// The tiles lie in shared memory row by row; the weight gradients, whose
+// reduction runs over the rows, read them with transposing ldmatrix loads
+// (transposed copies took 72 KB per block, 12 warps per SM and 2-byte stores at
+// 4-way bank conflicts: 221 us per launch at 262,144 cells, now 77).
+constexpr size_t BWD_SMEM = sizeof(bf16) * ((size_t)GNN_TILE * LDU       // sU: h, m
+                                            + (size_t)3 * GNN_TILE * LDH  // sDH, sA, sDZ
+                                            + (size_t)GNN_H * LDH         // sW2T
+                                            + (size_t)2 * GNN_H * LDH)    // sW1T
+                            + sizeof(float) * 8 * GNN_H;
 
-__global__ void __launch_bounds__(GNN_TILE) k_gnn_layer_bwd_mlp(GnnGraph g, TileLoop tl,
-                                                                const float *__restrict__ pl,
-                                                                const bf16 *__restrict__ pkl,
-                                                                const bf16 *__restrict__ hin0,
-                                                                const bf16 *__restrict__ a0p,
-                                                                const float *__restrict__ dho0,
-                                                                float *__restrict__ dhs0, float *__restrict__ dm0,
-                                                                float *__restrict__ gpart)
+__global__ void __launch_bounds__(BWD_THREADS, 3) k_gnn_layer_bwd_mlp(GnnGraph g, TileLoop tl,
+                                                                      const float *__restrict__ pl,
+                                                                      const bf16 *__restrict__ pkl,
+                                                                      const bf16 *__restrict__ hin0,
+                                                                      const bf16 *__restrict__ a0p,
+                                                                      const float *__restrict__ dho0,
+                                                                      float *__restrict__ dhs0,
+                                                                      float *__restrict__ dm0,
+                                                                      float *__restrict__ gpart)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    bf16 *sUT = reinterpret_cast<bf16 *>(smem);
-    bf16 *sDH = sUT + 2 * GNN_H * LDT;
-    bf16 *sDHT = sDH + GNN_TILE * LDH;
-    bf16 *sAT = sDHT + GNN_H * LDT;
-    bf16 *sDZ = sAT + GNN_H * LDT;
-    bf16 *sDZT = sDZ + GNN_TILE * LDH;
-    bf16 *sW2T = sDZT + GNN_H * LDT;
+    bf16 *sU = reinterpret_cast<bf16 *>(smem);
+    bf16 *sDH = sU + GNN_TILE * LDU;
+    bf16 *sA = sDH + GNN_TILE * LDH;
+    bf16 *sDZ = sA + GNN_TILE * LDH;
+    bf16 *sW2T = sDZ + GNN_TILE * LDH;
     bf16 *sW1T = sW2T + GNN_H * LDH;
     float(*red)[GNN_H] = reinterpret_cast<float(*)[GNN_H]>(sW1T + 2 * GNN_H * LDH);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = g.n;
-    for (int e = tid; e < GNN_H * GNN_H; e += GNN_TILE) sW2T[(e & 31) * LDH + (e >> 5)] = pkl[GKL_W2 + e];
-    for (int e = tid; e < GNN_H * 2 * GNN_H; e += GNN_TILE) sW1T[(e & 63) * LDH + (e >> 6)] = pkl[GKL_W1 + e];
-    const float wg0 = pl[GPL_WG + 2 * lane], wg1 = pl[GPL_WG + 2 * lane + 1], cg = pl[GPL_CG + lane];
-    const int gq = lane >> 2, tq = lane & 3;
-    const int mt0 = warp >> 1, nt2 = (warp & 1) * 2, nt1 = (warp & 1) * 4;
-    float s_dc2 = 0.f, dc1[4][2], accW2[1][2][4], accW1[1][4][4];
+    const int n = g.n, sub = lane >> 3, c4 = 4 * (lane & 7);
+    for (int e = tid; e < GNN_H * GNN_H; e += BWD_THREADS) sW2T[(e & 31) * LDH + (e >> 5)] = pkl[GKL_W2 + e];
+    for (int e = tid; e < GNN_H * 2 * GNN_H; e += BWD_THREADS) sW1T[(e & 63) * LDH + (e >> 6)] = pkl[GKL_W1 + e];
+    float wg0[4], wg1[4], cg[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        wg0[q] = pl[GPL_WG + 2 * (c4 + q)];
+        wg1[q] = pl[GPL_WG + 2 * (c4 + q) + 1];
+        cg[q] = pl[GPL_CG + c4 + q];
+    }
+    const int gq = lane >> 2, tq = lane & 3, mt = warp & 1, nq = warp >> 1;
+    // lane's row and column in the transposed 16 x 16 operand tiles
+    const int ta = ((lane >> 4) << 3) + (lane & 7), tc = ((lane >> 3) & 1) << 3;
+    const int ba = (((lane >> 3) & 1) << 3) + (lane & 7), bc = (lane >> 4) << 3;
+    float s_dc2[4] = {0.f, 0.f, 0.f, 0.f}, dc1[4][2], accW2[4] = {0.f, 0.f, 0.f, 0.f}, accW1[2][4];
 #pragma unroll
     for (int nt = 0; nt < 4; nt++) dc1[nt][0] = dc1[nt][1] = 0.f;
-    zero(accW2);
-    zero(accW1);
+#pragma unroll
+    for (int e = 0; e < 4; e++) accW1[0][e] = accW1[1][e] = 0.f;
     for (int tile = blockIdx.x; tile < tl.total; tile += gridDim.x) {
         const int y = tile / tl.ntiles, base = (tile - y * tl.ntiles) * GNN_TILE;
         const bf16 *hin = sample_rows(hin0, n, y), *a = sample_rows(a0p, n, y);
         const float *dho = sample_rows(dho0, n, y);
         float *dhs = sample_rows(dhs0, n, y), *dm = sample_rows(dm0, n, y);
-        const SlotCache mine = load_slots(g, base + warp * 32 + lane);
-        __syncthreads();  // the previous tile's products have read shared memory
-#pragma unroll 4
-        for (int r = 0; r < 32; r++) {
-            const int row = warp * 32 + r, i = base + row;
-            bf16 hi = __float2bfloat16(0.f), ai = hi;
-            float m = 0.f, d = 0.f;
+        __syncthreads();  // the previous tile's products have read shared memory (and the weights are there)
+#pragma unroll 1
+        for (int r = 0; r < 4; r++) {
+            const int row = warp * 16 + 4 * r + sub, i = base + row;
+            float4 h = make_float4(0.f, 0.f, 0.f, 0.f), av = h, d = h, m = h;
             if (i < n) {
-                hi = hin[(size_t)i * GNN_H + lane];
-                ai = a[(size_t)i * GNN_H + lane];
-                d = dho[(size_t)i * GNN_H + lane];
+                h = load_h4(hin + (size_t)i * GNN_H + c4);
+                av = load_h4(a + (size_t)i * GNN_H + c4);
+                d = *reinterpret_cast<const float4 *>(dho + (size_t)i * GNN_H + c4);
 #pragma unroll
                 for (int k = 0; k < 6; k++) {
-                    const int j = __shfl_sync(FULL, mine.col[k], r);
-                    const float2 e = edge_of(__shfl_sync(FULL, mine.edge[k], r));
-                    if (j != i) m += (wg0 * e.x + wg1 * e.y + cg) * __bfloat162float(hin[(size_t)j * GNN_H + lane]);
+                    const Slot4 sl = load_slot4(g, k, i, wg0, wg1, cg);
+                    const float4 hj = load_h4(hin + (size_t)sl.j * GNN_H + c4);
+                    if (sl.j != i) {
+                        m.x += sl.g[0] * hj.x;
+                        m.y += sl.g[1] * hj.y;
+                        m.z += sl.g[2] * hj.z;
+                        m.w += sl.g[3] * hj.w;
+                    }
                 }
             }
-            s_dc2 += d;
-            sUT[lane * LDT + row] = hi;
-            sUT[(GNN_H + lane) * LDT + row] = __float2bfloat16(m);
-            sAT[lane * LDT + row] = ai;
-            const bf16 db = __float2bfloat16(d);
-            sDH[row * LDH + lane] = db;
-            sDHT[lane * LDT + row] = db;
+            s_dc2[0] += d.x;
+            s_dc2[1] += d.y;
+            s_dc2[2] += d.z;
+            s_dc2[3] += d.w;
+            store_h4(sU + row * LDU + c4, h.x, h.y, h.z, h.w);
+            store_h4(sU + row * LDU + GNN_H + c4, m.x, m.y, m.z, m.w);
+            store_h4(sA + row * LDH + c4, av.x, av.y, av.z, av.w);
+            store_h4(sDH + row * LDH + c4, d.x, d.y, d.z, d.w);
+        }
+        __syncwarp();
+        float acc[1][4][4];
+        zero(acc);
+        warp_gemm16x32<2>(acc, sDH + warp * 16 * LDH, LDH, sW2T, LDH, lane);
+#pragma unroll
+        for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+            for (int hf = 0; hf < 2; hf++) {
+                const int row = warp * 16 + gq + 8 * hf, col = nt * 8 + 2 * tq;
+                const float2 a2 = __bfloat1622float2(*reinterpret_cast<const bf162 *>(sA + row * LDH + col));
+                const float z0 = a2.x > 0.f ? acc[0][nt][2 * hf] : 0.f;
+                const float z1 = a2.y > 0.f ? acc[0][nt][2 * hf + 1] : 0.f;
+                dc1[nt][0] += z0;
+                dc1[nt][1] += z1;
+                *reinterpret_cast<bf162 *>(sDZ + row * LDH + col) = __floats2bfloat162_rn(z0, z1);
+            }
+        __syncwarp();
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            zero(acc);
+            warp_gemm16x32<2>(acc, sDZ + warp * 16 * LDH, LDH, sW1T + half * GNN_H * LDH, LDH, lane);
+#pragma unroll
+            for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+                for (int hf = 0; hf < 2; hf++) {
+                    const int i = base + warp * 16 + gq + 8 * hf, col = nt * 8 + 2 * tq;
+                    if (i >= n) continue;
+                    float2 o = make_float2(acc[0][nt][2 * hf], acc[0][nt][2 * hf + 1]);
+                    if (half == 0) {
+                        const float2 d = *reinterpret_cast<const float2 *>(dho + (size_t)i * GNN_H + col);
+                        o.x += d.x;
+                        o.y += d.y;
+                    }
+                    *reinterpret_cast<float2 *>((half ? dm : dhs) + (size_t)i * GNN_H + col) = o;
+                }
         }
         __syncthreads();
-        {
-            float acc[2][4][4];
-            zero(acc);
-            warp_gemm<2, 4, 2>(acc, sDH + warp * 32 * LDH, LDH, sW2T, LDH, lane);
+        // dW2[o][in] += sum_cells dh'[cell][o] a[cell][in] (16 x 8 per warp);
+        // dW1[o][k] += sum_cells dz[cell][o] u[cell][k] (16 x 16 per warp)
 #pragma unroll
-            for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-                for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-                    for (int hf = 0; hf < 2; hf++) {
-                        const int row = warp * 32 + mt * 16 + gq + 8 * hf, col = nt * 8 + 2 * tq;
-                        const float a0 = __bfloat162float(sAT[col * LDT + row]);
-                        const float a1 = __bfloat162float(sAT[(col + 1) * LDT + row]);
-                        const float z0 = a0 > 0.f ? acc[mt][nt][2 * hf] : 0.f;
-                        const float z1 = a1 > 0.f ? acc[mt][nt][2 * hf + 1] : 0.f;
-                        dc1[nt][0] += z0;
-                        dc1[nt][1] += z1;
-                        const bf162 zb = __floats2bfloat162_rn(z0, z1);
-                        *reinterpret_cast<bf162 *>(sDZ + row * LDH + col) = zb;
-                        sDZT[col * LDT + row] = zb.x;
-                        sDZT[(col + 1) * LDT + row] = zb.y;
-                    }
+        for (int ks = 0; ks < GNN_TILE / 16; ks++) {
+            uint32_t fa[4], fb[4], b2[2];
+            ldm_x4_t(fa, sDH + (ks * 16 + ta) * LDH + mt * 16 + tc);
+            ldm_x2_t(b2, sA + (ks * 16 + (lane & 15)) * LDH + nq * 8);
+            mma_bf16(accW2, fa, b2);
+            ldm_x4_t(fa, sDZ + (ks * 16 + ta) * LDH + mt * 16 + tc);
+            ldm_x4_t(fb, sU + (ks * 16 + ba) * LDU + nq * 16 + bc);
+            const uint32_t b0[2] = {fb[0], fb[1]}, b1[2] = {fb[2], fb[3]};
+            mma_bf16(accW1[0], fa, b0);
+            mma_bf16(accW1[1], fa, b1);
         }
-        __syncthreads();
-        {
-            float acc[2][8][4];
-            zero(acc);
-            warp_gemm<2, 8, 2>(acc, sDZ + warp * 32 * LDH, LDH, sW1T, LDH, lane);
-#pragma unroll
-            for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-                for (int nt = 0; nt < 8; nt++)
-#pragma unroll
-                    for (int hf = 0; hf < 2; hf++) {
-                        const int row = warp * 32 + mt * 16 + gq + 8 * hf, col = nt * 8 + 2 * tq, i = base + row;
-                        if (i >= n) continue;
-                        if (nt < 4) {
-                            const float2 d = *reinterpret_cast<const float2 *>(dho + (size_t)i * GNN_H + col);
-                            *reinterpret_cast<float2 *>(dhs + (size_t)i * GNN_H + col) =
-                                make_float2(d.x + acc[mt][nt][2 * hf], d.y + acc[mt][nt][2 * hf + 1]);
-                        } else {
-                            *reinterpret_cast<float2 *>(dm + (size_t)i * GNN_H + col - GNN_H) =
-                                make_float2(acc[mt][nt][2 * hf], acc[mt][nt][2 * hf + 1]);
-                        }
-                    }
-        }
-        // dW2[o][in] += sum_cells dh'[cell][o] a[cell][in]; dW1[o][k] += sum_cells dz[cell][o] u[cell][k]
-        warp_gemm<1, 2, 8>(accW2, sDHT + mt0 * 16 * LDT, LDT, sAT + nt2 * 8 * LDT, LDT, lane);
-        warp_gemm<1, 4, 8>(accW1, sDZT + mt0 * 16 * LDT, LDT, sUT + nt1 * 8 * LDT, LDT, lane);
     }
     float *gp = gpart + (size_t)blockIdx.x * GNN_NPARAM;
 #pragma unroll
-    for (int nt = 0; nt < 2; nt++)
+    for (int hf = 0; hf < 2; hf++) {
+        const int o = mt * 16 + gq + 8 * hf;
+        gp[GPL_W2 + o * GNN_H + nq * 8 + 2 * tq] = accW2[2 * hf];
+        gp[GPL_W2 + o * GNN_H + nq * 8 + 2 * tq + 1] = accW2[2 * hf + 1];
 #pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-            const int o = mt0 * 16 + gq + 8 * hf, in = (nt2 + nt) * 8 + 2 * tq;
-            gp[GPL_W2 + o * GNN_H + in] = accW2[0][nt][2 * hf];
-            gp[GPL_W2 + o * GNN_H + in + 1] = accW2[0][nt][2 * hf + 1];
+        for (int nt = 0; nt < 2; nt++) {
+            const int k = nq * 16 + nt * 8 + 2 * tq;
+            gp[GPL_W1 + o * 2 * GNN_H + k] = accW1[nt][2 * hf];
+            gp[GPL_W1 + o * 2 * GNN_H + k + 1] = accW1[nt][2 * hf + 1];
         }
-#pragma unroll
-    for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-            const int o = mt0 * 16 + gq + 8 * hf, k = (nt1 + nt) * 8 + 2 * tq;
-            gp[GPL_W1 + o * 2 * GNN_H + k] = accW1[0][nt][2 * hf];
-            gp[GPL_W1 + o * 2 * GNN_H + k + 1] = accW1[0][nt][2 * hf + 1];
-        }
+    }
     // dc1: per-thread column sums -> over g lanes -> over warps
     __syncthreads();
 #pragma unroll
@@ -1059,59 +1125,78 @@ __global__ void __launch_bounds__(GNN_TILE) k_gnn_layer_bwd_mlp(GnnGraph g, Tile
             if (gq == 0) red[warp][nt * 8 + 2 * tq + e] = v;
         }
     __syncthreads();
-    if (warp == 0) gp[GPL_C1 + lane] = ((red[0][lane] + red[1][lane]) + red[2][lane]) + red[3][lane];
-    const float t_dc2 = block_channel_sum(s_dc2, red, warp, lane);
+    if (warp == 0) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; w++) t += red[w][lane];
+        gp[GPL_C1 + lane] = t;
+    }
+    const float t_dc2 = block_quad_sum(s_dc2, red, warp, lane);
     if (warp == 0) gp[GPL_C2 + lane] = t_dc2;
 }
 
 // Layer backward, message part: dh_in_j = dhs_j + sum over j's internal
-// slots of g (.) dm_other; partial gradients of Wg, cg.
-__global__ void __launch_bounds__(GNN_TILE) k_gnn_layer_bwd_msg(GnnGraph g, TileLoop tl,
-                                                                const float *__restrict__ pl,
-                                                                const bf16 *__restrict__ hin0,
-                                                                const float *__restrict__ dhs0,
-                                                                const float *__restrict__ dm0,
-                                                                float *__restrict__ dhi0, float *__restrict__ gpart)
+// slots of g (.) dm_other; partial gradients of Wg, cg.  Bound by its gathers
+// (six FP32 and six BF16 rows per cell, from L2): a warp has four rows, 12
+// row reads each, in flight per instruction (one row with a channel per lane
+// took 190 us per launch at 262,144 cells, now 67).
+__global__ void __launch_bounds__(BWD_THREADS, 4) k_gnn_layer_bwd_msg(GnnGraph g, TileLoop tl,
+                                                                      const float *__restrict__ pl,
+                                                                      const bf16 *__restrict__ hin0,
+                                                                      const float *__restrict__ dhs0,
+                                                                      const float *__restrict__ dm0,
+                                                                      float *__restrict__ dhi0,
+                                                                      float *__restrict__ gpart)
 {
-    __shared__ float red[4][GNN_H];
+    __shared__ float red[8][GNN_H];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n = g.n;
-    const float wg0 = pl[GPL_WG + 2 * lane], wg1 = pl[GPL_WG + 2 * lane + 1], cg = pl[GPL_CG + lane];
-    float s0 = 0.f, s1 = 0.f, sc = 0.f;
+    const int n = g.n, sub = lane >> 3, c4 = 4 * (lane & 7);
+    float wg0[4], wg1[4], cg[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        wg0[q] = pl[GPL_WG + 2 * (c4 + q)];
+        wg1[q] = pl[GPL_WG + 2 * (c4 + q) + 1];
+        cg[q] = pl[GPL_CG + c4 + q];
+    }
+    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, sc[4] = {0.f, 0.f, 0.f, 0.f};
     for (int tile = blockIdx.x; tile < tl.total; tile += gridDim.x) {
         const int y = tile / tl.ntiles, base = (tile - y * tl.ntiles) * GNN_TILE;
         const bf16 *hin = sample_rows(hin0, n, y);
         const float *dhs = sample_rows(dhs0, n, y), *dm = sample_rows(dm0, n, y);
         float *dhi = sample_rows(dhi0, n, y);
-        const SlotCache mine = load_slots(g, base + warp * 32 + lane);
-#pragma unroll 4
-        for (int r = 0; r < 32; r++) {
-            const int i = base + warp * 32 + r;
-            if (i < n) {  // (the same for every lane)
-                const float dmi = dm[(size_t)i * GNN_H + lane];
-                float acc = dhs[(size_t)i * GNN_H + lane];
+#pragma unroll 1
+        for (int r = 0; r < 4; r++) {
+            const int i = base + warp * 16 + 4 * r + sub;
+            if (i >= n) continue;
+            const float4 dv = *reinterpret_cast<const float4 *>(dm + (size_t)i * GNN_H + c4);
+            const float4 av = *reinterpret_cast<const float4 *>(dhs + (size_t)i * GNN_H + c4);
+            const float dmi[4] = {dv.x, dv.y, dv.z, dv.w};
+            float acc[4] = {av.x, av.y, av.z, av.w};
 #pragma unroll
-                for (int k = 0; k < 6; k++) {
-                    const int j = __shfl_sync(FULL, mine.col[k], r);
-                    const float2 e = edge_of(__shfl_sync(FULL, mine.edge[k], r));
-                    if (j != i) {
-                        acc += (wg0 * e.x + wg1 * e.y + cg) * dm[(size_t)j * GNN_H + lane];
-                        const float t = dmi * __bfloat162float(hin[(size_t)j * GNN_H + lane]);
-                        s0 += t * e.x;
-                        s1 += t * e.y;
-                        sc += t;
-                    }
+            for (int k = 0; k < 6; k++) {
+                const Slot4 sl = load_slot4(g, k, i, wg0, wg1, cg);
+                const float4 mj = *reinterpret_cast<const float4 *>(dm + (size_t)sl.j * GNN_H + c4);
+                const float4 hj = load_h4(hin + (size_t)sl.j * GNN_H + c4);
+                if (sl.j == i) continue;
+                const float mv[4] = {mj.x, mj.y, mj.z, mj.w}, hv[4] = {hj.x, hj.y, hj.z, hj.w};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    acc[q] += sl.g[q] * mv[q];
+                    const float t = dmi[q] * hv[q];
+                    s0[q] += t * sl.e.x;
+                    s1[q] += t * sl.e.y;
+                    sc[q] += t;
                 }
-                dhi[(size_t)i * GNN_H + lane] = acc;
             }
+            *reinterpret_cast<float4 *>(dhi + (size_t)i * GNN_H + c4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
         }
     }
     float *gp = gpart + (size_t)blockIdx.x * GNN_NPARAM;
-    const float t0 = block_channel_sum(s0, red, warp, lane);
+    const float t0 = block_quad_sum(s0, red, warp, lane);
     if (warp == 0) gp[GPL_WG + 2 * lane] = t0;
-    const float t1 = block_channel_sum(s1, red, warp, lane);
+    const float t1 = block_quad_sum(s1, red, warp, lane);
     if (warp == 0) gp[GPL_WG + 2 * lane + 1] = t1;
-    const float tc = block_channel_sum(sc, red, warp, lane);
+    const float tc = block_quad_sum(sc, red, warp, lane);
     if (warp == 0) gp[GPL_CG + lane] = tc;
 }
 
@@ -1389,9 +1474,9 @@ void gnn_loss_backward(cudaStream_t s, const GnnGraph &g, int samples, const Gnn
         const float *pl = p + GP_LAYER0 + l * GPL_SIZE;
         const bf16 *pkl = pk + GK_LAYER0 + l * GKL_SIZE;
         float *gpl = w.gpart + GP_LAYER0 + l * GPL_SIZE;
-        k_gnn_layer_bwd_mlp<<<nb, GNN_TILE, BWD_SMEM, s>>>(g, tl, pl, pkl, w.h[l], w.a[l], w.dh[cur], w.dh[cur ^ 1],
+        k_gnn_layer_bwd_mlp<<<nb, BWD_THREADS, BWD_SMEM, s>>>(g, tl, pl, pkl, w.h[l], w.a[l], w.dh[cur], w.dh[cur ^ 1],
                                                            w.dm, gpl);
-        k_gnn_layer_bwd_msg<<<nb, GNN_TILE, 0, s>>>(g, tl, pl, w.h[l], w.dh[cur ^ 1], w.dm, w.dh[cur], gpl);
+        k_gnn_layer_bwd_msg<<<nb, BWD_THREADS, 0, s>>>(g, tl, pl, w.h[l], w.dh[cur ^ 1], w.dm, w.dh[cur], gpl);
     }
     k_gnn_encode_bwd<<<nb, GNN_TILE, 0, s>>>(g, tl, batch, w.scales, w.h[0], w.dh[cur], w.gpart);
     k_gnn_reduce<<<(GNN_NPARAM + 31) / 32, 256, 0, s>>>(nb, w.gpart, grad);
