@@ -2472,7 +2472,9 @@ int mc_flow_create(const mc_mesh_view *mesh, const mc_flow_params *params, mc_fl
         }
     }
     if (!rc) {
-        cudaError_t e = cudaStreamSynchronize(h->stream);
+        // (some tables are copied on the default stream, which h->stream does not wait for)
+        cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
         if (e != cudaSuccess) rc = fail(h, MC_ERR_CUDA, cudaGetErrorString(e));
     }
     if (rc) {
@@ -2805,6 +2807,7 @@ int mc_flow_checkpoint_read(mc_flow *h, const char *path)
         CUDA_TRY(h, cudaMemcpy(arr.first, buf.data(), arr.second * 8, cudaMemcpyHostToDevice));
     }
     std::fclose(fp);
+    CUDA_TRY(h, cudaStreamSynchronize(cudaStreamLegacy));  // the copies, before kernels on h->stream read them
     h->timestep_count = hd.timestep_count;
     h->pass_in_step = hd.pass_in_step;
     h->first_pressure = hd.first_pressure;
@@ -2890,6 +2893,8 @@ int setup_nodes(mc_flow *h)
     CUDA_TRY(h, cudaMemcpy(h->pc_off, off.data(), (P + 1) * 4, cudaMemcpyHostToDevice));
     CUDA_TRY(h, cudaMemcpy(h->pc_cells, cells.data(), 8 * N * 4, cudaMemcpyHostToDevice));
     CUDA_TRY(h, cudaMemset(h->node_flag, 0, P));
+    // the tables were made on the default stream, which h->stream does not wait for
+    CUDA_TRY(h, cudaStreamSynchronize(cudaStreamLegacy));
     return MC_OK;
 }
 
