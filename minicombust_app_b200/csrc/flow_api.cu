@@ -131,7 +131,8 @@ struct mc_flow {
     double *partials;
     unsigned int *counter;
     FluxBalance *balance;
-    double *scalars;   // [0] max|PP|, [1] mass imbalance, [2] max |diag| of the pressure rows (FP16 level 0)
+    double *scalars;   // [0] max|PP|, [1] mass imbalance, [2] max |diag| of the pressure rows (FP16 level 0),
+                       // [3] total of device-resident mass sources, [4] max of the next corrector's right-hand side
     // Krylov
     PcgVectors pv{};
     BicgVectors<3> b3{};
@@ -239,7 +240,7 @@ struct mc_flow {
     int pass_in_step = 0;
     int sources_set = 0;
     double mass_source_total = 0.0;
-    bool mass_source_on_device = false;  // sources set from device memory: total in scalars[2]
+    bool mass_source_on_device = false;  // sources set from device memory: total in scalars[3]
     double p_bnorm_ref = 0.0;
     long launches = 0;
     Timing timing;
@@ -1084,7 +1085,7 @@ void launch_mass_flux(mc_flow *h)
     a.balance = h->balance;
     a.mass_source_total = (h->prm.mode == MC_MODE_SIMPLE && h->sources_set) ? h->mass_source_total : 0.0;
     a.mass_source_dev = (h->prm.mode == MC_MODE_SIMPLE && h->sources_set && h->mass_source_on_device)
-                            ? h->scalars + 2 : nullptr;
+                            ? h->scalars + 3 : nullptr;
     const int grid = std::min(blocks_for(h->F), krylov_grid(h->F));
     launch(h, K_MASS_FLUX, [&] { k_mass_flux<<<grid, MCB_THREADS, 0, h->stream>>>(h->ph, h->margs, a); });
     if (h->margs.n_outlet > 0)
@@ -2765,7 +2766,7 @@ int mc_flow_checkpoint_write(mc_flow *h, const char *path)
     hd.sources_set = h->sources_set;
     hd.mass_source_total = h->mass_source_total;
     if (h->mass_source_on_device)  // sources set from device memory: their total lives on the device
-        CUDA_TRY(h, cudaMemcpy(&hd.mass_source_total, h->scalars + 2, sizeof(double), cudaMemcpyDeviceToHost));
+        CUDA_TRY(h, cudaMemcpy(&hd.mass_source_total, h->scalars + 3, sizeof(double), cudaMemcpyDeviceToHost));
     bool ok = std::fwrite(&hd, sizeof(hd), 1, fp) == 1;
     std::vector<double> buf;
     for (const auto &arr : checkpoint_arrays(h)) {
@@ -3086,7 +3087,7 @@ int mc_flow_set_sources_device(mc_flow *h, const double *terms_soa)
     }
     launch(h, K_PERMUTE, [&] {
         k_sum<<<krylov_grid(h->N), MCB_THREADS, 0, h->stream>>>(h->N, h->src + 4 * N, h->partials, h->counter,
-                                                                h->scalars + 2);
+                                                                h->scalars + 3);
     });
     const int rc = check_launch(h);
     if (rc) return rc;
