@@ -303,7 +303,7 @@ const char *mc_status_string(int status);
  * and callers inside a time-critical loop, where cudaMalloc and cudaFree can
  * synchronise the device and stall the host's other streams.
  *
- * Solves A x = b with the BiCGStab kernels the temperature stage uses (zero
+ * Solves A x = b with the BiCGStab method the temperature stage uses (zero
  * initial guess, ||b - A x|| <= rtol ||b||), on a 7-point system the caller
  * owns on the current device, given in the ELL layout of this library:
  * diag[n], off[6][n], col[6][n] (an unused slot has col = its row, off = 0).
@@ -316,7 +316,9 @@ const char *mc_status_string(int status);
  * which keeps the last call's contents (each call clears what must start at
  * zero), so calls that overlap on the GPU race.  The first call on a device
  * looks up the array's address (cudaGetSymbolAddress, once per device, with
- * that device current).  iterations (may be NULL) receives the count. */
+ * that device current).  Up to 2,048 rows per SM the whole solve is one kernel;
+ * MC_ERR_TIMEOUT if its blocks waited for one another in vain.  iterations (may
+ * be NULL) receives the count. */
 #define MC_SOLVE_NOALLOC_MAX_ROWS 262144
 int mc_solve_bicgstab_noalloc(int n, const double *diag, const double *off, const int *col, const double *b,
                               double *x, double rtol, int max_iters, void *stream, int *iterations);

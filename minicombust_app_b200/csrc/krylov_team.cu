@@ -13,7 +13,14 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr int TEAM_THREADS = 1024;
+// Rows of a block up to which a thread holds one; above, two: their gathers
+// overlap and half as many warps are left to reduce (16,000 rows in 16 blocks:
+// 4.0 us per PCG iteration with one row per thread, 3.5 with two; four were no
+// faster).
+constexpr int TEAM_R1 = 256;
+// Threads of a block: at most 1024 rows in a cluster's blocks, 2048 in the grid's.
+template <bool CLUSTER, int RPT>
+constexpr int team_threads = RPT == 1 ? TEAM_R1 : CLUSTER ? 512 : 1024;
 constexpr int TEAM_CLUSTER = 16;      // blocks of the largest cluster
 constexpr unsigned TEAM_POLLS = 1u << 20;  // bound of a grid barrier's wait (about a second)
 
@@ -37,11 +44,10 @@ struct Team {
         const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
         const int buf = epoch & 1;
         epoch++;
+        warp_sums<K>(v, lane);
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-            v[k] = warp_sum_all(v[k]);
-            if (lane == 0) sw[k][warp] = v[k];
-        }
+        for (int k = 0; k < K; k++)
+            if (lane == ((k & 1) && k < (K & ~1) ? 16 : 0)) sw[k][warp] = v[k];
         __syncthreads();
         if (CLUSTER) {
             cg::cluster_group cl = cg::this_cluster();
@@ -113,14 +119,14 @@ size_t team_smem(int rows, int extra) { return (size_t)rows * (6 * 8 + 6 * 4 + 8
 
 // Rows of a block: thread t holds rows t, t + blockDim, ... of it (`RPT` of them).
 template <bool CLUSTER, int RPT>
-__global__ void __launch_bounds__(TEAM_THREADS, 1)
+__global__ void __launch_bounds__((team_threads<CLUSTER, RPT>), 1)
     k_pcg_team(Ell A, PcgVectors v, double rtol, double abs_floor, int max_iters, int use_x0, int rows, TeamMem m)
 {
     TEAM_SETUP;
     (void)se;
     double2 *__restrict__ zp = v.zp[0];
     const double mean = v.st->mean;
-    double x[RPT], r[RPT], z[RPT], p[RPT], d[RPT], q[RPT];
+    double x[RPT], r[RPT], z[RPT], p[RPT], d[RPT], di[RPT], q[RPT];
     bool on[RPT];
     double a3[3] = {0.0, 0.0, 0.0};  // b.b, r.z, r.r
 #pragma unroll
@@ -128,7 +134,7 @@ __global__ void __launch_bounds__(TEAM_THREADS, 1)
         const int l = t + e * nt, i = base + l;
         on[e] = l < rows && i < N;
         x[e] = r[e] = z[e] = p[e] = q[e] = 0.0;
-        d[e] = 1.0;
+        d[e] = di[e] = 1.0;
         if (!on[e]) continue;
         int c[6];
         row_cols(A, i, c);
@@ -147,7 +153,8 @@ __global__ void __launch_bounds__(TEAM_THREADS, 1)
         }
         const double bi = v.b[i] - mean;
         r[e] = use_x0 ? bi - ax : bi;
-        z[e] = d[e] != 0.0 ? r[e] / d[e] : r[e];
+        if (d[e] != 0.0) di[e] = 1.0 / d[e];  // a zero row (isolated cell) is left unpreconditioned
+        z[e] = r[e] * di[e];
         zp[i] = make_double2(z[e], 0.0);
         a3[0] += bi * bi;
         a3[1] += r[e] * z[e];
@@ -197,7 +204,7 @@ __global__ void __launch_bounds__(TEAM_THREADS, 1)
             if (!on[e]) continue;
             x[e] += alpha * p[e];
             r[e] -= alpha * q[e];
-            z[e] = d[e] != 0.0 ? r[e] / d[e] : r[e];
+            z[e] = r[e] * di[e];
             zp[base + t + e * nt] = make_double2(z[e], p[e]);
             a2[0] += r[e] * z[e];
             a2[1] += r[e] * r[e];
@@ -247,7 +254,7 @@ __global__ void __launch_bounds__(TEAM_THREADS, 1)
 }
 
 template <bool CLUSTER, int RPT>
-__global__ void __launch_bounds__(TEAM_THREADS, 1)
+__global__ void __launch_bounds__((team_threads<CLUSTER, RPT>), 1)
     k_bicg_team(Ell A, const double *__restrict__ b, double *__restrict__ xout, double2 *rp, double *vv0, double *vv1,
                 BicgState<1> *st, double rtol, int max_iters, int rows, TeamMem m)
 {
@@ -404,18 +411,18 @@ TeamShape team_shape(int N)
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return s;
-    if (N <= TEAM_CLUSTER * TEAM_THREADS) {
+    if (N <= TEAM_CLUSTER * 1024) {
         s.cluster = true;
         s.blocks = std::max(1, N / 128);
         if (s.blocks > 8) s.blocks = s.blocks >= TEAM_CLUSTER ? TEAM_CLUSTER : 8;
-    } else if (N <= sms * 2 * TEAM_THREADS) {
+    } else if (N <= sms * 2048) {
         s.blocks = sms;
     } else {
         return s;
     }
     s.rows = (N + s.blocks - 1) / s.blocks;
-    s.rpt = (s.rows + TEAM_THREADS - 1) / TEAM_THREADS;
-    s.threads = std::min(TEAM_THREADS, (s.rows + 31) / 32 * 32);
+    s.rpt = s.rows <= TEAM_R1 ? 1 : 2;
+    s.threads = ((s.rows + s.rpt - 1) / s.rpt + 31) / 32 * 32;
     return s;
 }
 
@@ -462,7 +469,8 @@ bool pcg_team(cudaStream_t s, const Ell &A, const PcgVectors &v, double rtol, do
     const TeamShape sh = team_shape(A.N);
     if (!sh.blocks) return false;
     const size_t smem = team_smem(sh.rows, 0);
-    auto k = sh.cluster ? k_pcg_team<true, 1> : (sh.rpt == 1 ? k_pcg_team<false, 1> : k_pcg_team<false, 2>);
+    auto k = sh.rpt == 1 ? (sh.cluster ? k_pcg_team<true, 1> : k_pcg_team<false, 1>)
+                         : (sh.cluster ? k_pcg_team<true, 2> : k_pcg_team<false, 2>);
     return team_launch(k, sh, smem, s, m, A, v, rtol, abs_floor, max_iters, use_x0, sh.rows, m);
 }
 
@@ -472,7 +480,8 @@ bool bicg_team(cudaStream_t s, const Ell &A, const double *b, double *x, double2
     const TeamShape sh = team_shape(A.N);
     if (!sh.blocks) return false;
     const size_t smem = team_smem(sh.rows, 2);
-    auto k = sh.cluster ? k_bicg_team<true, 1> : (sh.rpt == 1 ? k_bicg_team<false, 1> : k_bicg_team<false, 2>);
+    auto k = sh.rpt == 1 ? (sh.cluster ? k_bicg_team<true, 1> : k_bicg_team<false, 1>)
+                         : (sh.cluster ? k_bicg_team<true, 2> : k_bicg_team<false, 2>);
     return team_launch(k, sh, smem, s, m, A, b, x, rp, vv0, vv1, st, rtol, max_iters, sh.rows, m);
 }
 

@@ -106,6 +106,24 @@ __device__ __forceinline__ double warp_sum_all(double v)
     return v;
 }
 
+// Sums of K values over a warp.  The first step of a pair is shared: half the
+// warp keeps one value and sends the other, so two values take five exchanges
+// each way and not ten.  Result k is valid in lane 0 (k even) or 16 (k odd).
+template <int K>
+__device__ __forceinline__ void warp_sums(double (&v)[K], int lane)
+{
+#pragma unroll
+    for (int k = 0; k + 1 < K; k += 2) {
+        const bool hi = lane & 16;
+        const double keep = hi ? v[k + 1] : v[k], send = hi ? v[k] : v[k + 1];
+        double t = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        v[k] = v[k + 1] = t;
+    }
+    if (K & 1) v[K - 1] = warp_sum_all(v[K - 1]);
+}
+
 // Block sums of K values by warp shuffles (any block size that is a multiple
 // of 32): two barriers whatever K is.  sw: [K][32] shared; result in every
 // lane of warp 0.

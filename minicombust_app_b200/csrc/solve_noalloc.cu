@@ -2,9 +2,9 @@
 //
 // The handle-based solver keeps its Krylov vectors, block partials and status
 // block in the handle's cudaMalloc arena.  This entry point runs the same
-// kernels (k_bicg_init/1/2/3 with one right-hand side, as in the temperature
-// stage) on a system the caller owns, with every scratch byte taken from the
-// file-scope array below instead.  It exists for callers that must not
+// method as one kernel (krylov_team.cuh), or where no team of blocks holds the
+// rows as k_bicg_init/1/2/3 with one right-hand side, on a system the caller
+// owns, with every scratch byte taken from the file-scope array below instead.  It exists for callers that must not
 // allocate device memory: hosts that reserve all device memory for their own
 // pool or fixed budget at start-up (a library cudaMalloc would then fail, or
 // take memory the host has promised elsewhere), and callers inside a

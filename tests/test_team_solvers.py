@@ -1,6 +1,6 @@
 """Krylov solves run as one kernel by a team of blocks (cluster up to 16 x 1024
-rows, then a cooperative grid with one or two rows per thread), at the edges
-of the team's forms: BiCGStab through the allocation-free entry point, its
+rows, then a cooperative grid; one row per thread up to 256 rows a block, then
+two), at the edges of the team's forms: BiCGStab through the allocation-free entry point, its
 true residual checked in FP64 on the CPU, and the Jacobi-preconditioned
 pressure solve against the AMG-preconditioned one (the per-kernel solvers) on
 the same passes.
@@ -22,7 +22,7 @@ from minicombust_app_b200.workload import noisy_fields
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 31, 129, 1025, 2047, 2048, 9000, 16384, 16385, 151553, 262144])
+@pytest.mark.parametrize("n", [1, 31, 129, 1025, 2047, 2048, 4096, 4097, 9000, 16384, 16385, 151553, 262144])
 def test_bicgstab_team(gpu, n):
     import torch
     rng = np.random.default_rng(n)
