@@ -893,7 +893,7 @@ constexpr int SWEEP_MIN_ITERS = 50;
 // assembly 0.02 less without the FP32 rows), and their errors are 100 times smaller.
 bool sweeps_apply(const mc_flow *h)
 {
-    return h->line_ex > 0 && h->prm.max_iters >= SWEEP_MIN_ITERS && (!h->bir_mem || h->prm.ir_line_steps > 0);
+    return h->line64.ex > 0 && h->prm.max_iters >= SWEEP_MIN_ITERS && (!h->bir_mem || h->prm.ir_line_steps > 0);
 }
 
 template <int R>
@@ -1940,6 +1940,38 @@ int x_line_length(const std::vector<uint32_t> &code, const int doff[6], int N)
     return ex;
 }
 
+// Length of the x-lines of a reordered handle's caller (cell c of a line is
+// followed by cell c + 1 through its RIGHT face, in the caller's numbering), 0
+// where the caller's cells do not form lines of one length; `code` receives
+// the direction of each slot of each row (as DirCodes).
+int reordered_line_length(const HostMesh &hm, const std::vector<int> &o2n, std::vector<uint32_t> &code)
+{
+    const size_t N = (size_t)hm.N;
+    auto nbr = [&](int d, int i) { return hm.nbr[(size_t)d * N + i]; };
+    size_t ex = 0;
+    while (ex < N && nbr(RIGHT, o2n[ex]) >= 0) ex++;
+    ex++;
+    if (ex < 2 || ex > 1024 || N % ex != 0) return 0;
+    for (size_t c = 0; c < N; c++) {
+        const int i = o2n[c], r = nbr(RIGHT, i), l = nbr(LEFT, i);
+        if (c % ex != ex - 1 ? r != o2n[c + 1] : r >= 0) return 0;
+        if (c % ex != 0 ? l != o2n[c - 1] : l >= 0) return 0;
+    }
+    code.assign(N, 0u);
+    for (size_t i = 0; i < N; i++) {
+        uint32_t cw = 0;
+        for (int k = 0; k < 6; k++) {
+            const int j = hm.col[k * N + i];
+            unsigned d = 7;
+            for (unsigned q = 0; q < 6 && j != (int)i; q++)
+                if (nbr((int)q, (int)i) == j) d = q;
+            cw |= d << (3 * k);
+        }
+        code[i] = cw;
+    }
+    return (int)ex;
+}
+
 // Form of the pressure solvers' FP64 copy: 1 (default) the half form of the
 // symmetric matrix, 2 all six directions, 0 none (the slot-order matrix);
 // MC_PRESSURE_COPY overrides.  The FP32 level 0 keeps all six directions.
@@ -2413,6 +2445,23 @@ int mc_flow_create(const mc_mesh_view *mesh, const mc_flow_params *params, mc_fl
                             }
                         }
                     }
+                }
+            }
+            if (!rc && h->line64.ex == 0 && h->reordered) {
+                // the caller's x-lines in the handle's cell order
+                std::vector<uint32_t> code;
+                const int ex = reordered_line_length(hm, h->cell_o2n, code);
+                if (ex > 0) {
+                    LineRows64 &L = h->line64;
+                    L.N = (int)N;
+                    L.ex = ex;
+                    L.xm = LEFT;
+                    L.xp = RIGHT;
+                    L.code = h->dcode;
+                    L.perm = h->d_cell_o2n;
+                    L.col = h->col;
+                    rc = upload(h, h->dcode, code.data(), N);
+                    if (!rc) cudaStreamSynchronize(h->stream);
                 }
             }
             const int form = pressure_copy_form();

@@ -1239,10 +1239,18 @@ void bir_residual(cudaStream_t s, const Ell &A, const BirVectors<R> &v)
 // The residual of the iterate read is the right-hand side the map is formed
 // from less its own diagonal and -x terms, so convergence costs no extra pass
 // over the matrix; the iterate returned is one sweep better than the one tested.
-template <int R, bool DIR>
+// Forms of the rows: by position, in slot order with direction codes, or the
+// latter in another cell order than the lines' (LineRows64::perm).  There the
+// rows of a line are gathered (they stay near one another in a bandwidth-
+// reducing order) and the neighbours are read through the columns, 28 bytes of
+// index per row more: still four sweeps where BiCGStab takes 8 to 10
+// iterations, a pass on 524,000 reordered cells 8.16 -> 6.87 ms.
+enum { LINE_POS = 0, LINE_SLOT = 1, LINE_PERM = 2 };
+
+template <int FORM>
 __device__ __forceinline__ double line_value(const LineRows64 &L, size_t i, uint32_t cw, int d)
 {
-    if (DIR) return L.off[(size_t)d * L.N + i];
+    if (FORM == LINE_POS) return L.off[(size_t)d * L.N + i];
     double v = 0.0;
 #pragma unroll
     for (int k = 0; k < 6; k++)
@@ -1262,7 +1270,7 @@ constexpr int sweep_lines = R == 1 ? 8 : 3;
 template <int R>
 constexpr int sweep_blocks = R == 1 ? 5 : 4;
 
-template <int R, bool DIR, bool FIRST>
+template <int R, int FORM, bool FIRST>
 __global__ void __launch_bounds__(32 * R * sweep_lines<R>, sweep_blocks<R>)
     k_line_sweep64(LineRows64 L, SweepVectors<R> v, SweepPtrs<R> x, int to, double rtol)
 {
@@ -1281,32 +1289,50 @@ __global__ void __launch_bounds__(32 * R * sweep_lines<R>, sweep_blocks<R>)
         const int base = line * ex;
         double carry = 0.0, xlast = 0.0;  // e and x of the cell before the chunk
         for (int c0 = 0; c0 < ex; c0 += 32) {
-            const int c = c0 + lane, i = base + min(c, ex - 1);
+            const int c = c0 + lane, at = base + min(c, ex - 1), i = FORM == LINE_PERM ? L.perm[at] : at;
             const bool on = c < ex;
-            const uint32_t cw = DIR ? 0u : L.code[i];
+            const uint32_t cw = FORM == LINE_POS ? 0u : L.code[i];
             const double d = L.diag[i];
-            const double a = line_value<R, DIR>(L, i, cw, L.xm);
+            double a = 0.0;
+            if (FORM != LINE_PERM || FIRST) a = line_value<FORM>(L, i, cw, L.xm);
             double s = b[i];
             if (FIRST) {
                 if (on) sum += s * s;
             } else {
                 const double x0 = xin[i];
-                double xe = 0.0;  // the cell after the chunk's last
-                if (lane == 31 && c + 1 < ex) xe = xin[i + 1];
-                const double op = line_value<R, DIR>(L, i, cw, L.xp);
-                double o[4], xy[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    o[u] = line_value<R, DIR>(L, i, cw, L.yz[u]);
-                    xy[u] = xin[min(max(i + L.yzoff[u], 0), N - 1)];
-                }
-                double xp = __shfl_down_sync(0xffffffffu, x0, 1), xm = __shfl_up_sync(0xffffffffu, x0, 1);
-                if (lane == 31) xp = xe;
+                double xm = __shfl_up_sync(0xffffffffu, x0, 1);
                 if (lane == 0) xm = xlast;
                 xlast = __shfl_sync(0xffffffffu, x0, 31);
-                if (c + 1 < ex) s -= op * xp;
+                if (FORM == LINE_PERM) {
+                    double o[6], xc[6];
 #pragma unroll
-                for (int u = 0; u < 4; u++) s -= o[u] * xy[u];
+                    for (int k = 0; k < 6; k++) {
+                        o[k] = L.off[(size_t)k * N + i];
+                        xc[k] = xin[L.col[(size_t)k * N + i]];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 6; k++) {
+                        if (((cw >> (3 * k)) & 7u) == (unsigned)L.xm)
+                            a = o[k];
+                        else
+                            s -= o[k] * xc[k];
+                    }
+                } else {
+                    double xe = 0.0;  // the cell after the chunk's last
+                    if (lane == 31 && c + 1 < ex) xe = xin[i + 1];
+                    const double op = line_value<FORM>(L, i, cw, L.xp);
+                    double o[4], xy[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        o[u] = line_value<FORM>(L, i, cw, L.yz[u]);
+                        xy[u] = xin[min(max(i + L.yzoff[u], 0), N - 1)];
+                    }
+                    double xp = __shfl_down_sync(0xffffffffu, x0, 1);
+                    if (lane == 31) xp = xe;
+                    if (c + 1 < ex) s -= op * xp;
+#pragma unroll
+                    for (int u = 0; u < 4; u++) s -= o[u] * xy[u];
+                }
                 double res = s - d * x0;
                 if (c > 0) res -= a * xm;
                 if (on) sum += res * res;
@@ -1359,7 +1385,7 @@ __global__ void __launch_bounds__(32 * R * sweep_lines<R>, sweep_blocks<R>)
 }
 
 namespace {
-template <int R, bool DIR, bool FIRST>
+template <int R, int FORM, bool FIRST>
 void launch_line_sweep64(cudaStream_t s, const LineRows64 &L, const SweepVectors<R> &v, int from, double rtol)
 {
     constexpr int LB = sweep_lines<R>;
@@ -1371,7 +1397,7 @@ void launch_line_sweep64(cudaStream_t s, const LineRows64 &L, const SweepVectors
         x.in[j] = v.x[from][j];
         x.out[j] = v.x[from ^ 1][j];
     }
-    pdl_launch(k_line_sweep64<R, DIR, FIRST>, dim3(grid), dim3(32 * R * LB), 0, s, L, v, x, from ^ 1, rtol);
+    pdl_launch(k_line_sweep64<R, FORM, FIRST>, dim3(grid), dim3(32 * R * LB), 0, s, L, v, x, from ^ 1, rtol);
 }
 } // namespace
 
@@ -1380,12 +1406,15 @@ int line_sweep64_blocks(int N) { return krylov_grid(N); }
 template <int R>
 void line_sweep64(cudaStream_t s, const LineRows64 &L, const SweepVectors<R> &v, int k, double rtol)
 {
-    if (L.code)
-        k == 0 ? launch_line_sweep64<R, false, true>(s, L, v, 0, rtol)
-               : launch_line_sweep64<R, false, false>(s, L, v, k & 1, rtol);
+    if (L.perm)
+        k == 0 ? launch_line_sweep64<R, LINE_PERM, true>(s, L, v, 0, rtol)
+               : launch_line_sweep64<R, LINE_PERM, false>(s, L, v, k & 1, rtol);
+    else if (L.code)
+        k == 0 ? launch_line_sweep64<R, LINE_SLOT, true>(s, L, v, 0, rtol)
+               : launch_line_sweep64<R, LINE_SLOT, false>(s, L, v, k & 1, rtol);
     else
-        k == 0 ? launch_line_sweep64<R, true, true>(s, L, v, 0, rtol)
-               : launch_line_sweep64<R, true, false>(s, L, v, k & 1, rtol);
+        k == 0 ? launch_line_sweep64<R, LINE_POS, true>(s, L, v, 0, rtol)
+               : launch_line_sweep64<R, LINE_POS, false>(s, L, v, k & 1, rtol);
 }
 template void line_sweep64<1>(cudaStream_t, const LineRows64 &, const SweepVectors<1> &, int, double);
 template void line_sweep64<3>(cudaStream_t, const LineRows64 &, const SweepVectors<3> &, int, double);

@@ -272,8 +272,8 @@ struct BirVectors {
 
 // FP64 x-line sweeps: the whole momentum or transport solve as the splitting
 // iteration x_{k+1} = M^-1 (b - (A - M) x_k), M the diagonal and the -x
-// couplings of each x-line, from x_0 = 0, on a structured box whose cells run
-// x-fastest along whole lines.  Each sweep also forms the true residual of
+// couplings of each x-line, from x_0 = 0, on a mesh whose cells run x-fastest
+// along whole lines, in that order or renumbered.  Each sweep also forms the true residual of
 // the iterate it reads.
 struct LineRows64 {
     int N = 0;
@@ -283,6 +283,10 @@ struct LineRows64 {
     int yzoff[4] = {0, 0, 0, 0};
     const uint32_t *code = nullptr;  // null: off rows are positions; else slot order with these direction codes
                                      // (xm, xp and yz are then directions)
+    // cells not in line order (reordered handles): the row of cell c of line l
+    // is perm[l ex + c], and the columns [6][N] are read too (code is set)
+    const int *perm = nullptr;
+    const int *col = nullptr;
     const double *diag = nullptr;
     const double *off = nullptr;     // [6][N]
 };

@@ -1,7 +1,7 @@
 """The FP64 x-line sweeps (momentum, temperature and scalar solves on boxes
 whose cells run x-fastest) against the CPU oracle, whose solves are BiCGStab:
-line lengths at the edges of the 32-cell scan chunks and of the shared-memory
-split, meshes of a few lines, and a flow across the lines with a long time
+line lengths at the edges of the 32-cell scan chunks, meshes of a few lines,
+handles that renumber their cells, and a flow across the lines with a long time
 step, where the splitting converges too slowly and BiCGStab takes over.
 
 Solves run to 1e-12 on both sides; fields agree to 1e-9 of their maximum, the
@@ -48,6 +48,12 @@ def run_both(dims, passes=2, base=BASE, **kw):
 def test_sweeps_match_oracle(gpu, dims):
     st = run_both(dims)
     # a sweep gains about three decades on this flow: 1e-12 within one batch
+    assert 1 <= max(st.momentum_iters) <= 12 and 1 <= st.temperature_iters <= 12
+
+
+@pytest.mark.parametrize("dims", [(2, 3, 3), (32, 2, 5), (33, 5, 3), (257, 2, 2), (18, 17, 9)])
+def test_renumbered_sweeps_match_oracle(gpu, dims):
+    st = run_both(dims, reorder=1, transport_scalars=1)
     assert 1 <= max(st.momentum_iters) <= 12 and 1 <= st.temperature_iters <= 12
 
 
