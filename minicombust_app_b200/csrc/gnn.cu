@@ -1415,7 +1415,7 @@ static void forward_impl(cudaStream_t s, const GnnGraph &g, const GnnBatch<T> &i
             const bf16 *wf = w.fold + (size_t)l * 7 * GNN_H * GNN_H;
             if (umma)
                 gnn_layer_umma(s, g, maps[l & 1], pl, wf, pkl, w.h[l & 1], w.h[(l + 1) & 1], w.status, sm_count(),
-                               l == GNN_L - 1 ? &dec : nullptr);
+                               l == GNN_L - 1 ? &dec : nullptr, l > 0);
             else
                 k_gnn_layer_fold<<<std::min(nb, sm_count()), LAYER_THREADS, FOLD_SMEM, s>>>(
                     g, pl, wf, pkl, w.h[l & 1], w.h[(l + 1) & 1], nb);

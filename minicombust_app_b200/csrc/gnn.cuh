@@ -171,9 +171,12 @@ struct GnnUmmaDecode {
 };
 // One offset-form layer on the tcgen05 tensor cores, `grid` persistent
 // blocks, hin (described by `map`) -> hout, or with dec the network's output.
+// weights_ready: wf was complete before the kernel launched before this one
+// (a layer after the first), so it is read while that one drains.
 void gnn_layer_umma(cudaStream_t s, const GnnGraph &g, const GnnTmaMap &map, const float *pl,
                     const __nv_bfloat16 *wf, const __nv_bfloat16 *pkl, const __nv_bfloat16 *hin,
-                    __nv_bfloat16 *hout, int *status, int grid, const GnnUmmaDecode *dec = nullptr);
+                    __nv_bfloat16 *hout, int *status, int grid, const GnnUmmaDecode *dec = nullptr,
+                    bool weights_ready = false);
 
 // Training: forward, loss against `target` (units of the solution), backward
 // of up to w.samples samples; adds their gradients, scaled by `weight`, into

@@ -290,8 +290,9 @@ int mc_gnn_predict(mc_gnn *net, const mc_gnn_graph *gr, const mc_gnn_sample *s, 
     GNN_TRY(cudaSetDevice(net->dev));
     int rc = ensure_work(net, gr->g.n, 0);
     if (rc) return rc;
-    gnn_forward<float>(net->stream, gr->g, input_of(*s), net->p, net->pk, net->work, x0);
-    if (y) GNN_TRY(cudaMemcpyAsync(y, net->work.y, (size_t)gr->g.n * 4, cudaMemcpyDeviceToDevice, net->stream));
+    GnnWork work = net->work;
+    if (y) work.y = y;  // the prediction is written where the caller wants it
+    gnn_forward<float>(net->stream, gr->g, input_of(*s), net->p, net->pk, work, x0);
     GNN_TRY(cudaGetLastError());
     int status = 0;
     GNN_TRY(cudaMemcpyAsync(&status, net->work.status, sizeof(int), cudaMemcpyDeviceToHost, net->stream));
