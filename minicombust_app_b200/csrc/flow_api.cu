@@ -2982,14 +2982,15 @@ int mc_flow_ingest_particles(mc_flow *h, int64_t rows, const uint64_t *cells, co
         rc = check_launch(h);
         if (rc) return rc;
     }
-    // the total mass source, summed in the caller's cell order as mc_flow_set_sources does
-    std::vector<double> fuel(N);
-    CUDA_TRY(h, cudaMemcpyAsync(fuel.data(), h->src + 4 * N, N * 8, cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    double total = 0.0;
-    for (size_t i = 0; i < N; i++) total += fuel[h->reordered ? (size_t)h->cell_o2n[i] : i];
-    h->mass_source_total = total;
-    h->mass_source_on_device = false;
+    // the total mass source stays on the device (as for mc_flow_set_sources_device)
+    launch(h, K_EXCHANGE, [&] {
+        k_sum<<<krylov_grid(h->N), MCB_THREADS, 0, h->stream>>>(h->N, h->src + 4 * N, h->partials, h->counter,
+                                                                h->scalars + 3);
+    });
+    const int rs = check_launch(h);
+    if (rs) return rs;
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));  // the caller's rows may go
+    h->mass_source_on_device = true;
     h->sources_set = 1;
     return MC_OK;
 }

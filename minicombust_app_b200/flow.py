@@ -375,14 +375,14 @@ class FlowSolver:
         """(node ids ascending, [nodes][5] = vel.x, vel.y, vel.z, pressure, temp)
         for the nodes of the given cells."""
         c = np.ascontiguousarray(cells, dtype=np.uint64)
+        # room for every node there can be, so that one call finds and fills them
+        most = min(8 * c.shape[0], self.mesh.points.shape[0])
         n = ctypes.c_int64()
-        _check(self.L.mc_flow_interpolate_nodes(self.h, c.shape[0], _ptr(c), 0, ctypes.byref(n), None, None),
-               self.h, "interpolate_nodes")
-        ids = np.empty(n.value, dtype=np.uint64)
-        vals = np.empty((n.value, 5))
-        _check(self.L.mc_flow_interpolate_nodes(self.h, c.shape[0], _ptr(c), n.value, ctypes.byref(n), _ptr(ids),
+        ids = np.empty(most, dtype=np.uint64)
+        vals = np.empty((most, 5))
+        _check(self.L.mc_flow_interpolate_nodes(self.h, c.shape[0], _ptr(c), most, ctypes.byref(n), _ptr(ids),
                                                 _ptr(vals)), self.h, "interpolate_nodes")
-        return ids, vals
+        return ids[:n.value], vals[:n.value]
 
     def face_array(self, which):
         width = {4: 2, 5: 3, 6: 3}.get(which, 1)

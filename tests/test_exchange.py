@@ -96,3 +96,24 @@ def test_ingest_many_rows_and_reuse(gpu):
     with pytest.raises(flow.FlowError) as e:
         s.ingest_particles(np.array([s.N], dtype=np.uint64), np.zeros((1, 5)))
     assert e.value.status == flow.MC_ERR_ARG
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("reorder", [flow.REORDER_NONE, flow.REORDER_RCM], ids=["natural", "rcm"])
+def test_ingest_run_lengths(gpu, reorder):
+    """Cells that receive 1 to 25 rows and one that receives 3,000, the last
+    run ending with the rows: each sum bitwise that of its rows in arrival order
+    (the device adds them in batches of eight)."""
+    s = flow.FlowSolver(flow.Mesh.box(9, 5, 4, 0.2, 0.1, 0.1),
+                        params=flow.default_params(flow.MODE_SIMPLE, reorder=reorder))
+    rng = np.random.default_rng(8)
+    counts = {7 * k % s.N: k for k in range(1, 26)}
+    for last in (1, 8, 9, 3000):
+        counts[s.N - 1] = last
+        cells = rng.permutation(np.repeat(np.array(list(counts), dtype=np.uint64), list(counts.values())))
+        rows = rng.standard_normal((cells.shape[0], 5))
+        s.ingest_particles(cells, rows)
+        want = np.zeros((s.N, 5))
+        np.add.at(want, cells.astype(np.int64), rows)
+        assert np.array_equal(s.sources(), want), last
+    s.close()
