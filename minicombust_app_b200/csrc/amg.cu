@@ -182,6 +182,35 @@ int amg_build_host(int N, const std::vector<int> &col0, const std::vector<int> &
     return -1;
 }
 
+void amg_mark_boxes(std::vector<AmgHostLevel> &lv, int nx, int ny, int nz)
+{
+    for (size_t l = 0; l + 1 < lv.size(); l++) {
+        AmgHostLevel &L = lv[l];
+        if (nx < 2 || ny < 2 || nz < 2 || (long)nx * ny * nz != L.n) return;
+        // neighbours only across the faces of the box's cells
+        if (l > 0 && !(L.dia && L.doff[0] == -nx * ny && L.doff[1] == -nx && L.doff[2] == -1 && L.doff[3] == 1 &&
+                       L.doff[4] == nx && L.doff[5] == nx * ny))
+            return;
+        const int cx = (nx + 1) / 2, cy = (ny + 1) / 2, cz = (nz + 1) / 2;
+        for (int i = 0; i < L.n; i++) {
+            const int x = i % nx, y = (i / nx) % ny, z = i / (nx * ny);
+            if (L.agg[i] != ((z / 2) * cy + y / 2) * cx + x / 2) return;
+            for (int s = 0; s < L.k; s++) {
+                const int j = L.col[(size_t)s * L.n + i];
+                if (j == i) continue;
+                const int dx = abs(j % nx - x), dy = abs((j / nx) % ny - y), dz = abs(j / (nx * ny) - z);
+                if (dx + dy + dz != 1) return;
+            }
+        }
+        L.box[0] = nx;
+        L.box[1] = ny;
+        L.box[2] = nz;
+        nx = cx;
+        ny = cy;
+        nz = cz;
+    }
+}
+
 // ------------------------------------------------------------------ kernels
 
 namespace {
@@ -637,6 +666,12 @@ __global__ void __launch_bounds__(AMG_FUSED_THREADS)
     }
 }
 
+} // namespace mcb
+
+#include "amg_tile.cuh"
+
+namespace mcb {
+
 // ------------------------------------------------------------------ drivers
 
 namespace {
@@ -720,11 +755,82 @@ void amg_plan_fused(AmgHierarchy &H)
 // the saved passes).
 bool amg_paired_sweeps(const AmgHierarchy &H, bool fp32) { return fp32 && H.sweeps >= 2; }
 
+// Blocks of the tile kernels the device holds: one (FP32: two) per SM.
+template <typename T>
+static long tile_resident()
+{
+    return (long)krylov_grid(INT32_MAX - 256) / 8 * (sizeof(T) == 4 ? 2 : 1);
+}
+
+// Split of a box level into tile columns and planes: the one whose waves of
+// resident blocks take the fewest steps (a block of zc planes takes zc + 7).
+struct TilePlan {
+    int zc = 0;
+    long blocks = 0, steps = 0;
+};
+template <typename T>
+static TilePlan tile_plan(const int box[3])
+{
+    const long cols = (long)((box[0] + TILE_UX - 1) / TILE_UX) * ((box[1] + TILE_UY - 1) / TILE_UY);
+    const long resident = tile_resident<T>();
+    TilePlan best;
+    for (int c = 1; c <= std::max(1, box[2] / 4); c++) {
+        const int zc = ((box[2] + c - 1) / c + 1) & ~1;
+        const long blocks = cols * ((box[2] + zc - 1) / zc), steps = (blocks + resident - 1) / resident * (zc + 7);
+        if (best.zc == 0 || steps < best.steps) best = {zc, blocks, steps};
+    }
+    return best;
+}
+
+// The tile kernels pay where their steps, overlap and idle blocks included, are
+// few per row.  V-cycles by sweeps and with tiles at six box sizes, FP64: 2.44
+// cell steps per row 321 -> 261 us (256 x 128 x 128), 2.57 249 -> 227 (128^3),
+// 3.03 234 -> 228 (320 x 64 x 100), 3.32 84 -> 76 (128 x 64 x 64), 3.44 118 ->
+// 118 (160 x 80 x 80), above that slower.  FP32 sweeps stream half the bytes:
+// 2.57 231 -> 188, 2.82 151 -> 153, 3.03 150 -> 160.
+template <typename T>
+bool amg_tile_fits(const int box[3], int sweeps, int form)
+{
+    if (form == 0 || sweeps != 3 || box[0] == 0) return false;
+    const double rows = (double)box[0] * box[1] * box[2], waste = sizeof(T) == 8 ? 3.35 : 2.7;
+    const TilePlan p = tile_plan<T>(box);
+    // one partial sum per block, of the 24 per kernel grid block the solvers have
+    if (p.blocks > 24L * krylov_grid((int)rows)) return false;
+    return form == 2 || (double)p.steps * tile_resident<T>() * TILE_T <= waste * rows;
+}
+template bool amg_tile_fits<double>(const int *, int, int);
+template bool amg_tile_fits<float>(const int *, int, int);
+
 // Per level above the fused ones: nu sweeps before and after the coarse
-// correction and the restriction.
+// correction and the restriction, or the two tile kernels.
 int amg_kernels_per_vcycle(const AmgHierarchy &H, bool fp32)
 {
-    return H.fused_from * (2 * H.sweeps + (amg_paired_sweeps(H, fp32) ? 0 : 2)) + 1;
+    int n = 1;
+    for (int l = 0; l < H.fused_from; l++)
+        n += (fp32 ? H.lv32[l].box[0] : H.lv[l].box[0]) > 0
+                 ? 2
+                 : 2 * H.sweeps + (amg_paired_sweeps(H, fp32) ? 0 : 2);
+    return n;
+}
+
+// Half a V-cycle on a box level: down (rc, e out) or up (ec; e in, eout or zp).
+template <typename T, bool UP>
+static void launch_tile(cudaStream_t s, const AmgLevelT<T> &V, TileArgs<T> a)
+{
+    a.L.nx = V.box[0];
+    a.L.ny = V.box[1];
+    a.L.nz = V.box[2];
+    a.L.diag = V.diag;
+    a.L.cx = V.off + (size_t)V.plus[0] * V.n;
+    a.L.cy = V.off + (size_t)V.plus[1] * V.n;
+    a.L.cz = V.off + (size_t)V.plus[2] * V.n;
+    a.r = V.r;
+    const int gx = (a.L.nx + TILE_UX - 1) / TILE_UX, gy = (a.L.ny + TILE_UY - 1) / TILE_UY;
+    a.zc = tile_plan<T>(V.box).zc;
+    const dim3 grid(gx, gy, (a.L.nz + a.zc - 1) / a.zc);
+    constexpr size_t smem = tile_smem<T, UP>();
+    cudaFuncSetAttribute(k_amg_tile<T, UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    pdl_launch(k_amg_tile<T, UP>, grid, dim3(TILE_T), smem, s, a);
 }
 
 template <typename T>
@@ -750,6 +856,16 @@ void amg_vcycle(cudaStream_t s, const AmgHierarchy &H, const T *r0, void *zp_out
         const dim3 g(blocks(V.n));
         const bool hv = h0 && l == 0;
         int c = 0, sw = 1;
+        if (V.box[0] > 0) {
+            TileArgs<T> a{};
+            for (int k = 0; k < 3; k++) a.w[k] = w(k);
+            a.e = V.e[0];
+            a.rc = lv[l + 1].r;
+            a.st = st;
+            launch_tile<T, false>(s, V, a);
+            cur[l] = 0;
+            continue;
+        }
         if (pair) {
             pdl_launch(hv ? k_amg_smooth_first2<T, true> : k_amg_smooth_first2<T, false>, g, nt, 0, s, V, w(0), w(1),
                        V.e[1], st);
@@ -779,6 +895,22 @@ void amg_vcycle(cudaStream_t s, const AmgHierarchy &H, const T *r0, void *zp_out
         const bool hv = h0 && l == 0;
         const T *ec = lv[l + 1].e[cur[l + 1]];
         int c = cur[l], sw = 1;
+        if (V.box[0] > 0) {
+            TileArgs<T> a{};
+            for (int k = 0; k < 3; k++) a.w[k] = w(2 - k);
+            a.e = V.e[c];
+            a.ec = ec;
+            a.alpha = alpha;
+            a.eout = V.e[c ^ 1];
+            a.zp = l == 0 ? zp_out : nullptr;
+            a.st = st;
+            a.partials = partials;
+            a.counter = counter;
+            a.is_init = is_init;
+            launch_tile<T, true>(s, V, a);
+            cur[l] = c ^ 1;
+            continue;
+        }
         if (pair) {
             pdl_launch(hv ? k_amg_prolong_jacobi<T, true> : k_amg_prolong_jacobi<T, false>, g, nt, 0, s, V,
                        w(H.sweeps - 1), alpha, ec, V.e[c], V.e[c ^ 1], st);

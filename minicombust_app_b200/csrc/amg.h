@@ -66,6 +66,10 @@ struct AmgLevelT {
     // Null: every kernel reads off.
     __half *off16 = nullptr;
     float *scale16 = nullptr;
+    // sizes of a level whose halves of the V-cycle run as one kernel each (0:
+    // not so), and the rows of off that hold its +x, +y and +z couplings
+    int box[3] = {0, 0, 0};
+    int plus[3] = {0, 0, 0};
 };
 using AmgLevel = AmgLevelT<double>;
 
@@ -109,10 +113,21 @@ struct AmgHostLevel {
     // columns), with value 0 and column = row where the row has none.
     int dia = 0;
     int doff[6] = {0, 0, 0, 0, 0, 0};
+    // sizes of a box in x-fastest order whose aggregates are the 2 x 2 x 2
+    // blocks at even coordinates (0: not such a level)
+    int box[3] = {0, 0, 0};
 };
 
 int amg_build_host(int N, const std::vector<int> &col0, const std::vector<int> &dn0, std::vector<AmgHostLevel> &out,
                    std::string &err);
+
+// Mark the levels that are boxes with the sizes nx, ny, nz of level 0 halved
+// (rounded up) from level to level and 2 x 2 x 2 aggregates (AmgHostLevel::box).
+void amg_mark_boxes(std::vector<AmgHostLevel> &lv, int nx, int ny, int nz);
+// Whether a box level's halves of the V-cycle run as one kernel each: form 0
+// never, 1 where that is faster, 2 on every box.
+template <typename T>
+bool amg_tile_fits(const int box[3], int sweeps, int form);
 
 // Device work, all asynchronous on stream s.
 // Galerkin values of levels 1..L-1 for the FP64 (T = double) or the FP32

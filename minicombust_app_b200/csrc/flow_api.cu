@@ -1981,6 +1981,14 @@ int pressure_copy_form()
     return (v && *v) ? std::atoi(v) : 1;
 }
 
+// Tile kernels of the V-cycle (amg_tile_fits): 1 (default) where they are
+// faster, 0 none, 2 on every box; MC_AMG_TILES overrides.
+int amg_tile_form()
+{
+    const char *v = std::getenv("MC_AMG_TILES");
+    return (v && *v) ? std::atoi(v) : 1;
+}
+
 bool dir_codes_disabled()
 {
     const char *v = std::getenv("MC_DIR_CODES");
@@ -2082,6 +2090,13 @@ int build_amg(mc_flow *h, const HostMesh &hm)
     std::vector<AmgHostLevel> lv;
     std::string err;
     if (amg_build_host(N, hm.col, dn, lv, err) != 0) return fail(h, MC_ERR_MESH, err);
+    // the box's sizes, where the cells are one in x-fastest order
+    if (h->line_ex > 0) {
+        int plane = 0;
+        for (int d = 0; d < 6; d++) plane = std::max(plane, h->dc.doff[d]);
+        if (plane > h->line_ex && plane % h->line_ex == 0 && N % plane == 0)
+            amg_mark_boxes(lv, h->line_ex, plane / h->line_ex, N / plane);
+    }
     const int L = (int)lv.size();
     if (L < 2) {  // the whole system is already at the coarsest size: plain Jacobi PCG
         h->use_amg = false;
@@ -2126,8 +2141,11 @@ int build_amg(mc_flow *h, const HostMesh &hm)
     add(&H.dense_next, (size_t)nc * nc * 8);
     const bool fp32 = h->prm.precision == MC_PRECISION_FP32_REFINED;
     PcgState *inner_state = nullptr;
-    // the FP16 copy of the FP32 level 0 (values by direction) for the V-cycle
-    const bool half0 = fp32 && h->dc.code && !amg_half_disabled();
+    // the FP16 copy of the FP32 level 0 (values by direction) for the V-cycle's
+    // sweeps; the tile kernels read the FP32 values once per half
+    const int tiles = amg_tile_form();
+    const bool half0 =
+        fp32 && h->dc.code && !amg_half_disabled() && !amg_tile_fits<float>(lv[0].box, H.sweeps, tiles);
     if (fp32) {
         for (int l = 0; l < L; l++) {
             AmgLevelT<float> &f = H.lv32[l];
@@ -2192,6 +2210,20 @@ int build_amg(mc_flow *h, const HostMesh &hm)
             d.mlist = d_mlist[l];
         }
     }
+    // levels of the tile kernels, and the rows of off with their +x, +y and +z couplings
+    auto mark = [&](auto &d, const AmgHostLevel &a, bool fits) {
+        const int step[3] = {1, a.box[0], a.box[0] * a.box[1]};
+        if (!fits || !d.dc.dia) return;
+        for (int q = 0; q < 3; q++) {
+            int row = -1;
+            for (int k = 0; k < 6; k++)
+                if (d.dc.doff[k] == step[q]) row = d.dc.sym ? k >> 1 : k;
+            if (row < 0) return;
+            d.plus[q] = row;
+        }
+        for (int q = 0; q < 3; q++) d.box[q] = a.box[q];
+    };
+    for (int l = 0; l < L; l++) mark(H.lv[l], lv[l], amg_tile_fits<double>(lv[l].box, H.sweeps, tiles));
     H.g0 = H.lv[0];  // the slot-order level 0 (Galerkin lists, FP32 rounding)
     H.g0.off = h->off_p;
     H.g0.dc = h->dc;
@@ -2208,6 +2240,7 @@ int build_amg(mc_flow *h, const HostMesh &hm)
             f.mlist = d.mlist;
             f.gptr = d.gptr;
             f.gidx = d.gidx;
+            mark(f, lv[l], amg_tile_fits<float>(lv[l].box, H.sweeps, tiles));
         }
         h->pv32.b = h->r32;
         h->pv32.partials = h->partials;

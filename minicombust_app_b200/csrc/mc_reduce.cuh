@@ -147,7 +147,8 @@ __device__ __forceinline__ void block_sums(double (&v)[K], double (*sw)[32])
 // publish_partials / reduce_partials with shuffle sums.
 template <int K>
 __device__ __forceinline__ bool publish_sums(const double (&v)[K], double *partials, unsigned int *counter,
-                                             double (*sw)[32])
+                                             double (*sw)[32], unsigned int block = blockIdx.x,
+                                             unsigned int blocks = gridDim.x)
 {
     __shared__ bool am_last;
     double b[K];
@@ -156,9 +157,9 @@ __device__ __forceinline__ bool publish_sums(const double (&v)[K], double *parti
     block_sums<K>(b, sw);
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int k = 0; k < K; k++) partials[(size_t)blockIdx.x * K + k] = b[k];
+        for (int k = 0; k < K; k++) partials[(size_t)block * K + k] = b[k];
         __threadfence();
-        am_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        am_last = atomicAdd(counter, 1u) == blocks - 1;
     }
     __syncthreads();
     return am_last;
@@ -168,11 +169,11 @@ __device__ __forceinline__ bool publish_sums(const double (&v)[K], double *parti
 // takes blocks t, t + blockDim, ...).  Result in thread 0.
 template <int K>
 __device__ __forceinline__ void reduce_sums(double (&out)[K], const double *partials, unsigned int *counter,
-                                            double (*sw)[32])
+                                            double (*sw)[32], unsigned int blocks = gridDim.x)
 {
 #pragma unroll
     for (int k = 0; k < K; k++) out[k] = 0.0;
-    for (unsigned int b = threadIdx.x; b < gridDim.x; b += blockDim.x)
+    for (unsigned int b = threadIdx.x; b < blocks; b += blockDim.x)
 #pragma unroll
         for (int k = 0; k < K; k++) out[k] += __ldcg(partials + (size_t)b * K + k);
     block_sums<K>(out, sw);

@@ -1,0 +1,66 @@
+"""V-cycle halves as one kernel per level (MC_AMG_TILES=2: every box level of the
+hierarchy) against the per-sweep kernels (0): the same operator in another
+order of evaluation.  Boxes at the edges of the tiles (26 x 10 cells, even plane
+counts) and of the levels' halving: one cell over or under, odd sizes, two cells.
+
+The pressure solve stops at 1e-2 of its right-hand side, so a V-cycle that
+differed anywhere would change the fields by about 1e-2 of the correction: more
+than 1e-5 of the pressure here.  Rounding leaves 1e-9 of each field (FP64) and,
+with the FP32 V-cycle inside, 1e-6.
+"""
+import os
+
+import numpy as np
+import pytest
+
+from minicombust_app_b200 import flow
+from minicombust_app_b200.workload import noisy_fields
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("U", "V", "W", "P", "TEM")
+
+
+def run(dims, tiles, **kw):
+    saved = os.environ.get("MC_AMG_TILES"), os.environ.get("MC_AMG_HALF")
+    os.environ.update(MC_AMG_TILES=tiles, MC_AMG_HALF="0")
+    try:
+        s = flow.FlowSolver(flow.Mesh.box(*dims, 0.2, 0.1, 0.1),
+                            params=flow.default_params(flow.MODE_SIMPLE, pressure_solver=flow.PSOLVER_PCG_AMG,
+                                                       p_rtol=1e-2, **kw))
+    finally:
+        for k, v in zip(("MC_AMG_TILES", "MC_AMG_HALF"), saved):
+            os.environ.pop(k, None) if v is None else os.environ.update({k: v})
+    for name, vals in noisy_fields(s.N, seed=3).items():
+        a = s.field(name)
+        a[:s.N] = vals
+        s.set_field(name, a)
+    its = []
+    for _ in range(2):
+        s.simple_iteration()
+        its.append(s.last_stats.as_dict()["pressure_iters_total"])
+    fields = {n: s.field(n) for n in FIELDS}
+    s.close()
+    return fields, its
+
+
+@pytest.mark.parametrize("dims", [(26, 10, 8), (27, 11, 7), (52, 20, 9), (53, 21, 33), (25, 9, 31), (2, 30, 40),
+                                  (104, 2, 20), (40, 40, 2), (40, 41, 3), (79, 31, 65)])
+@pytest.mark.parametrize("fp32", [False, True], ids=["fp64", "fp32"])
+def test_tiles_match_sweeps(gpu, dims, fp32):
+    kw = dict(precision=flow.PRECISION_FP32_REFINED) if fp32 else {}
+    tiles, its_t = run(dims, "2", **kw)
+    sweeps, its_s = run(dims, "0", **kw)
+    assert its_t == its_s
+    for n in FIELDS:
+        rel = np.abs(tiles[n] - sweeps[n]).max() / np.abs(sweeps[n]).max()
+        assert rel <= (1e-6 if fp32 else 1e-9), (n, rel)
+
+
+def test_rule_takes_tiles_at_a_large_box(gpu):
+    """At 256 x 128 x 128 the default rule tiles levels 0 and 1."""
+    rule, its_r = run((256, 128, 128), "1")
+    sweeps, its_s = run((256, 128, 128), "0")
+    assert its_r == its_s
+    for n in FIELDS:
+        assert np.abs(rule[n] - sweeps[n]).max() <= 1e-9 * np.abs(sweeps[n]).max(), n
