@@ -182,11 +182,18 @@ int amg_build_host(int N, const std::vector<int> &col0, const std::vector<int> &
     return -1;
 }
 
-void amg_mark_boxes(std::vector<AmgHostLevel> &lv, int nx, int ny, int nz)
+void amg_mark_boxes(std::vector<AmgHostLevel> &lv, int nx, int ny, int nz, int sweeps, int form)
 {
     for (size_t l = 0; l + 1 < lv.size(); l++) {
         AmgHostLevel &L = lv[l];
         if (nx < 2 || ny < 2 || nz < 2 || (long)nx * ny * nz != L.n) return;
+        const int size[3] = {nx, ny, nz};
+        if (!amg_tile_fits<double>(size, sweeps, form) && !amg_tile_fits<float>(size, sweeps, form)) {
+            nx = (nx + 1) / 2;
+            ny = (ny + 1) / 2;
+            nz = (nz + 1) / 2;
+            continue;
+        }
         // neighbours only across the faces of the box's cells
         if (l > 0 && !(L.dia && L.doff[0] == -nx * ny && L.doff[1] == -nx && L.doff[2] == -1 && L.doff[3] == 1 &&
                        L.doff[4] == nx && L.doff[5] == nx * ny))

@@ -123,7 +123,8 @@ int amg_build_host(int N, const std::vector<int> &col0, const std::vector<int> &
 
 // Mark the levels that are boxes with the sizes nx, ny, nz of level 0 halved
 // (rounded up) from level to level and 2 x 2 x 2 aggregates (AmgHostLevel::box).
-void amg_mark_boxes(std::vector<AmgHostLevel> &lv, int nx, int ny, int nz);
+// Only the levels that amg_tile_fits takes are looked at.
+void amg_mark_boxes(std::vector<AmgHostLevel> &lv, int nx, int ny, int nz, int sweeps, int form);
 // Whether a box level's halves of the V-cycle run as one kernel each: form 0
 // never, 1 where that is faster, 2 on every box.
 template <typename T>

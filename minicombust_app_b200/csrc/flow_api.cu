@@ -2091,11 +2091,12 @@ int build_amg(mc_flow *h, const HostMesh &hm)
     std::string err;
     if (amg_build_host(N, hm.col, dn, lv, err) != 0) return fail(h, MC_ERR_MESH, err);
     // the box's sizes, where the cells are one in x-fastest order
+    const int tiles = amg_tile_form();
     if (h->line_ex > 0) {
         int plane = 0;
         for (int d = 0; d < 6; d++) plane = std::max(plane, h->dc.doff[d]);
         if (plane > h->line_ex && plane % h->line_ex == 0 && N % plane == 0)
-            amg_mark_boxes(lv, h->line_ex, plane / h->line_ex, N / plane);
+            amg_mark_boxes(lv, h->line_ex, plane / h->line_ex, N / plane, h->prm.amg_sweeps, tiles);
     }
     const int L = (int)lv.size();
     if (L < 2) {  // the whole system is already at the coarsest size: plain Jacobi PCG
@@ -2143,7 +2144,6 @@ int build_amg(mc_flow *h, const HostMesh &hm)
     PcgState *inner_state = nullptr;
     // the FP16 copy of the FP32 level 0 (values by direction) for the V-cycle's
     // sweeps; the tile kernels read the FP32 values once per half
-    const int tiles = amg_tile_form();
     const bool half0 =
         fp32 && h->dc.code && !amg_half_disabled() && !amg_tile_fits<float>(lv[0].box, H.sweeps, tiles);
     if (fp32) {
