@@ -9,7 +9,7 @@
 // reduction (block partials, a counter, the last block's second pass) -- 5 to
 // 7 us a kernel however few the rows.  A team's sum costs 1.1 us (cluster of
 // 16) or 2.5 us (148 blocks).  Measured, before and after: Jacobi PCG 14 -> 3.5
-// us per iteration at 16,000 rows and 23 -> 9.5 us at 221,000; BiCGStab 20 ->
+// us per iteration at 16,000 rows and 23 -> 8.5 us at 221,000; BiCGStab 20 ->
 // 5.2 us at 3,000 rows and 29 -> 16 us at 262,000.
 #pragma once
 
