@@ -2480,8 +2480,11 @@ int mc_flow_create(const mc_mesh_view *mesh, const mc_flow_params *params, mc_fl
                     }
                 }
             }
-            if (!rc && h->line64.ex == 0 && h->reordered) {
-                // the caller's x-lines in the handle's cell order
+            if (!rc && h->line64.ex == 0 && h->reordered && !h->dc.code) {
+                // The caller's x-lines in the handle's cell order.  Rows in
+                // slot order only: with direction codes (renumbering can keep
+                // them, e.g. a mesh of one line reversed) the rows are stored
+                // by position and dcode is theirs.
                 std::vector<uint32_t> code;
                 const int ex = reordered_line_length(hm, h->cell_o2n, code);
                 if (ex > 0) {

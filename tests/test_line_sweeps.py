@@ -51,6 +51,14 @@ def test_sweeps_match_oracle(gpu, dims):
     assert 1 <= max(st.momentum_iters) <= 12 and 1 <= st.temperature_iters <= 12
 
 
+@pytest.mark.parametrize("dims", [(2, 1, 1), (33, 1, 1), (1000, 1, 1), (1, 33, 1)])
+@pytest.mark.parametrize("reorder", [0, 1], ids=["natural", "rcm"])
+def test_single_lines_match_oracle(gpu, dims, reorder):
+    """A mesh of one line: renumbering reverses it, so that its rows are stored
+    by direction although the handle's own order has no x-lines."""
+    run_both(dims, reorder=reorder, transport_scalars=1)
+
+
 @pytest.mark.parametrize("dims", [(2, 3, 3), (32, 2, 5), (33, 5, 3), (257, 2, 2), (18, 17, 9)])
 def test_renumbered_sweeps_match_oracle(gpu, dims):
     st = run_both(dims, reorder=1, transport_scalars=1)
