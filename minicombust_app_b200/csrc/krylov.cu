@@ -476,7 +476,8 @@ __global__ void __launch_bounds__(MCB_THREADS) k_guess_apply(int N, double *__re
 // evaluated at each row where the product needs it and stored in xout (not
 // in x, which neighbouring rows still read); without e, x' = x.  r may be
 // null (the FP64 residual is then not stored).
-// With alt set x and xout change places when st->iter is odd (ir_residual_alt).
+// With alt set x and xout change places when st->iter is odd, and an inner solve
+// that broke down ends the refinement at the x it started from (ir_residual_alt).
 __global__ void __launch_bounds__(MCB_THREADS) k_ir_residual(Ell A, const double *__restrict__ b, const double *x0,
                                                              const float *__restrict__ e, double *x1,
                                                              double *__restrict__ r, float *__restrict__ r32,
@@ -486,6 +487,15 @@ __global__ void __launch_bounds__(MCB_THREADS) k_ir_residual(Ell A, const double
     pdl_wait();
     __shared__ double sh[1][MCB_THREADS];
     const int N = A.N;
+    if (inner && inner->status == KRYLOV_NONFINITE) {
+        // (every block returns here, so none sees the state written below)
+        if (blockIdx.x == 0 && threadIdx.x == 0 && !st->done) {
+            st->inner_total += inner->iter;
+            st->done = 1;
+            st->status = KRYLOV_NONFINITE;
+        }
+        return;
+    }
     const bool odd = alt && (st->iter & 1);
     const double *__restrict__ x = odd ? x1 : x0;
     double *__restrict__ xout = odd ? const_cast<double *>(x0) : x1;

@@ -395,7 +395,9 @@ void guess_apply(cudaStream_t s, int N, double *x, const double *xa, const doubl
 void ir_residual(cudaStream_t s, const Ell &A, const double *b, const double *x, double *r, float *r32, PcgState *st,
                  double *partials, unsigned int *counter, const float *e = nullptr, double *xout = nullptr);
 // The same inside a device loop: the solution alternates between x and x2 by
-// the parity of st->iter (x first), and inner's iterations are added up.
+// the parity of st->iter (x first), and inner's iterations are added up.  An
+// inner solve that ended KRYLOV_NONFINITE ends the refinement with that status,
+// its result not added.
 void ir_residual_alt(cudaStream_t s, const Ell &A, const double *b, double *x, double *x2, float *r32, PcgState *st,
                      double *partials, unsigned int *counter, const float *e, const PcgState *inner);
 // x2 (may be null): the solution is there when st->iter is odd.
