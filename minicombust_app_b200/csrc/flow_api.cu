@@ -1096,8 +1096,9 @@ void launch_mass_flux(mc_flow *h)
 }
 
 // The corrections of one corrector: the correction's gradient, the face
-// fluxes, then the cells (with the next corrector's right-hand side in simple mode).
-void launch_corrections(mc_flow *h, int simple, int cell0)
+// fluxes, then the cells (with the next corrector's right-hand side in simple
+// mode).  skip: as CorrectArgs::skip.
+void launch_corrections(mc_flow *h, int simple, int cell0, const int *skip = nullptr)
 {
     launch_gradient_pressure(h, G_PP);
     CorrectArgs c{};
@@ -1113,6 +1114,7 @@ void launch_corrections(mc_flow *h, int simple, int cell0)
     c.fcorr = h->fcorr;
     c.next_rhs = simple ? h->b_p : nullptr;
     c.rhs_max = simple ? h->scalars + 4 : nullptr;
+    c.skip = skip;
     const int grid_f = std::min(blocks_for(h->F), krylov_grid(h->F));
     launch(h, K_PP_FACES, [&] { launch_pp_correct_faces(h->stream, grid_f, h->ortho, h->ph, h->margs, c); });
     launch(h, K_PP_CELLS,
@@ -1181,8 +1183,9 @@ bool corrector_graph(mc_flow *h, int use_x0)
                 });
             }
             pcg_xmean(h->stream, h->N, v, x2);
-            pcg_finish(h->stream, h->N, v, x2, h->pp_prev, h->ph.cell0, h->scalars, h->scalars + 4);
-            launch_corrections(h, 1, 0);
+            pcg_finish(h->stream, h->N, v, x2, h->pp_prev, h->ph.cell0, h->scalars, h->scalars + 4,
+                       h->prm.initial_guess == MC_GUESS_LEARNED && use_x0 ? h->gs : nullptr);
+            launch_corrections(h, 1, 0, &v.st->skip);
             ok = cudaMemcpyAsync(h->h_pcg, v.st, sizeof(PcgState), cudaMemcpyDeviceToHost, h->stream) == cudaSuccess && ok;
             ok = cudaMemcpyAsync(h->h_scalars, h->scalars, 5 * sizeof(double), cudaMemcpyDeviceToHost, h->stream) ==
                      cudaSuccess && ok;
@@ -1426,7 +1429,8 @@ int stage_pressure(mc_flow *h, mc_iter_stats *st)
                 st->pressure_rel_residual = std::max(st->pressure_rel_residual, relres);
                 st->pressure_correction_max_first = pc_ref;
             }
-            if (!std::isfinite(pc_ref)) return fail(h, MC_ERR_NONFINITE, "pressure correction is not finite");
+            if (ps.status == KRYLOV_NONFINITE || !std::isfinite(pc_ref))
+                return fail(h, MC_ERR_NONFINITE, "pressure correction is not finite");
             more = pc_ref > 0.25 * pc_ref;
             // A zero right-hand side (orthogonal faces: no flux correction)
             // solves to zero: the second corrector would only leave the

@@ -1098,6 +1098,7 @@ __global__ void __launch_bounds__(MCB_THREADS) k_face_offsets(int N, MeshArgs m,
 template <bool ORTHO>
 __global__ void __launch_bounds__(MCB_THREADS, 4) k_pp_correct_faces(Physics ph, MeshArgs m, CorrectArgs a)
 {
+    if (a.skip && *a.skip) return;
     const int N = ph.N, F = m.F;
     for (int face = grid_stride_start(); face < F; face += gridDim.x * blockDim.x) {
         const int c0 = m.fc0[face], c1 = m.fc1[face];
@@ -1127,6 +1128,7 @@ template <bool ORTHO>
 __global__ void __launch_bounds__(MCB_THREADS, 4) k_pp_correct_cells(Physics ph, MeshArgs m, CorrectArgs a,
                                                                   int correct_all, int correct_cell0)
 {
+    if (a.skip && *a.skip) return;
     const int N = ph.N;
     const int c = grid_stride_start();
     double rmax = 0.0;

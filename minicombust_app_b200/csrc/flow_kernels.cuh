@@ -133,6 +133,7 @@ struct CorrectArgs {
     double *mdot, *fcorr;
     double *next_rhs;           // null: do not build the next corrector's right-hand side
     double *rhs_max;            // max |next_rhs| (zero before the launch); null: not formed
+    const int *skip;            // nonzero: nothing is corrected; null: always corrected
 };
 
 // The gradient kernel is a template; it is launched from its own translation

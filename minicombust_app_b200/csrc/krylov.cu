@@ -562,16 +562,18 @@ __global__ void __launch_bounds__(MCB_THREADS) k_pcg_sub_xmean(int N, PcgVectors
 
 __global__ void __launch_bounds__(MCB_THREADS) k_pcg_finish(int N, PcgVectors v, const double *x2,
                                                             double *__restrict__ prev, int cell0, double *pp_max,
-                                                            double *zero)
+                                                            double *zero, const GuessState *gs)
 {
     __shared__ double sh[1][MCB_THREADS];
+    const bool skip = v.st->status == KRYLOV_NONFINITE || (gs && gs->net_status);
+    if (blockIdx.x == 0 && threadIdx.x == 0) v.st->skip = skip;
     const double m = v.st->xmean;
     const double *x = (x2 && (v.st->iter & 1)) ? x2 : v.x;
     double acc[1] = {-1.0e308};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         const double xi = x[i] - m;
         v.x[i] = xi;
-        prev[i] = xi;
+        if (!skip) prev[i] = xi;
         acc[0] = fmax(acc[0], i == cell0 ? xi : fabs(xi));
     }
     if (publish_partials<1, true>(acc, v.partials, v.counter, sh)) {
@@ -655,9 +657,9 @@ void pcg_xmean(cudaStream_t s, int N, const PcgVectors &v, const double *x2)
     k_pcg_xmean<<<krylov_grid(N), MCB_THREADS, 0, s>>>(N, v, x2);
 }
 void pcg_finish(cudaStream_t s, int N, const PcgVectors &v, const double *x2, double *prev, int cell0, double *pp_max,
-                double *zero)
+                double *zero, const GuessState *gs)
 {
-    k_pcg_finish<<<krylov_grid(N), MCB_THREADS, 0, s>>>(N, v, x2, prev, cell0, pp_max, zero);
+    k_pcg_finish<<<krylov_grid(N), MCB_THREADS, 0, s>>>(N, v, x2, prev, cell0, pp_max, zero, gs);
 }
 void pcg_sub_xmean(cudaStream_t s, int N, const PcgVectors &v)
 {

@@ -209,6 +209,7 @@ struct PcgState {
     double rz, rz_old, alpha, pq, rr, bb, tol2, mean, xmean;
     int iter, done, status, max_iters;
     int inner_total;  // refinement: iterations of the inner solves so far
+    int skip;         // pcg_finish: the solution is not to be applied
 };
 
 template <int R>
@@ -404,9 +405,11 @@ void ir_residual_alt(cudaStream_t s, const Ell &A, const double *b, double *x, d
 void pcg_xmean(cudaStream_t s, int N, const PcgVectors &v, const double *x2 = nullptr);
 void pcg_sub_xmean(cudaStream_t s, int N, const PcgVectors &v);
 // v.x = solution - mean, its copy in prev, and the largest correction (as
-// k_pp_max) in *pp_max; *zero = 0 for the kernel that follows.
+// k_pp_max) in *pp_max; *zero = 0 for the kernel that follows.  After a solve
+// that ended KRYLOV_NONFINITE, or with a guess whose network gave up (gs, may
+// be null), prev is left as it was and v.st->skip set, else cleared.
 void pcg_finish(cudaStream_t s, int N, const PcgVectors &v, const double *x2, double *prev, int cell0, double *pp_max,
-                double *zero);
+                double *zero, const GuessState *gs);
 
 template <typename T, int R>
 void bicg_init_t(cudaStream_t s, const EllT<T> &A, const BicgVectorsT<T, R> &v, double rtol, int max_iters);
