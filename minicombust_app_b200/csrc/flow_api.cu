@@ -608,10 +608,6 @@ int after_pressure_solve(mc_flow *h)
 
 int launch_deferred_inverse(mc_flow *h);
 
-// Barrier memory of the team solvers: a word of the counters' block and the
-// block partials (a team runs alone on the handle's stream).
-TeamMem team_mem(mc_flow *h) { return TeamMem{h->counter + 16, h->partials}; }
-
 int solve_pressure(mc_flow *h, double abs_floor, int *iters, double *relres, double *bnorm)
 {
     const Ell A = pressure_matrix(h);
@@ -625,7 +621,7 @@ int solve_pressure(mc_flow *h, double abs_floor, int *iters, double *relres, dou
         // small systems: the whole solve in one kernel
         bool team = false;
         launch(h, K_PCG_TEAM, [&] {
-            team = pcg_team(h->stream, A, v, h->prm.p_rtol, abs_floor, h->prm.max_iters, use_x0, team_mem(h));
+            team = pcg_team(h->stream, A, v, h->prm.p_rtol, abs_floor, h->prm.max_iters, use_x0);
         });
         if (team) {
             CUDA_TRY(h, cudaMemcpyAsync(h->h_pcg, v.st, sizeof(PcgState), cudaMemcpyDeviceToHost, h->stream));
@@ -635,7 +631,7 @@ int solve_pressure(mc_flow *h, double abs_floor, int *iters, double *relres, dou
             *iters = s.iter;
             *bnorm = std::sqrt(s.bb);
             *relres = s.bb > 0 ? std::sqrt(s.rr / s.bb) : 0.0;
-            return krylov_status_to_mc(s.status);
+            return krylov_status_to_mc(team_status(s, s.status));
         }
         h->launches--;
     }
@@ -824,15 +820,15 @@ int solve_bicg(mc_flow *h, const Ell &A, const BicgVectors<R> &v, BicgState<R> *
     if constexpr (R == 1) {  // small systems: the whole solve in one kernel
         bool team = false;
         launch(h, K_BICG1_TEAM, [&] {
-            team = bicg_team(h->stream, A, v.b, v.x[0], h->pv.zp[0], v.v[0], v.v[1], v.st, h->prm.u_rtol,
-                             h->prm.max_iters, team_mem(h));
+            team = bicg_team(h->stream, A, v.b, v.x[0], h->pv.zp[0], v.v[0], v.v[1], v.partials, v.st,
+                             h->prm.u_rtol, h->prm.max_iters);
         });
         if (team) {
             CUDA_TRY(h, cudaMemcpyAsync(hs, v.st, sizeof(BicgState<R>), cudaMemcpyDeviceToHost, h->stream));
             CUDA_TRY(h, cudaStreamSynchronize(h->stream));
             flush_timing(h);
             iters_out[0] = hs->iter[0];
-            return krylov_status_to_mc(hs->status[0]);
+            return krylov_status_to_mc(team_status(*hs, hs->status[0]));
         }
         h->launches--;
     }
@@ -1450,7 +1446,7 @@ int stage_pressure(mc_flow *h, mc_iter_stats *st)
         h->corrector = loop;
         rc = h->refined ? solve_pressure_refined(h, floor, &its, &relres, &bnorm)
                         : solve_pressure(h, floor, &its, &relres, &bnorm);
-        if (rc == MC_ERR_CUDA) return rc;
+        if (rc == MC_ERR_CUDA || rc == MC_ERR_TIMEOUT) return rc;  // (no solution to correct with)
         if (rc != MC_OK && worst == MC_OK) worst = rc;
         if (loop == 1) h->p_bnorm_ref = bnorm;
         {
@@ -1603,7 +1599,7 @@ int stage_scalar(mc_flow *h, int field, mc_iter_stats *st)
     if (!solve_rc && !swept)
         solve_rc =
             solve_bicg<1>(h, temperature_matrix(h), h->bs, h->h_b1, &h->g_bs, &h->l_bs, K_BICG1_INIT, K_BICG1_1, its);
-    if (solve_rc == MC_ERR_CUDA) return solve_rc;
+    if (solve_rc == MC_ERR_CUDA || solve_rc == MC_ERR_TIMEOUT) return solve_rc;
     CUDA_TRY(h, cudaMemcpyAsync(phi, h->xs, (size_t)h->N * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
     if (type == SC_TERBTE || type == SC_TERBED) {
         ClipArgs c{};

@@ -210,6 +210,7 @@ struct PcgState {
     int iter, done, status, max_iters;
     int inner_total;  // refinement: iterations of the inner solves so far
     int skip;         // pcg_finish: the solution is not to be applied
+    unsigned int team[2];  // team solvers (krylov_team.cuh): arrivals; nonzero: a block's wait ran out
 };
 
 template <int R>
@@ -217,6 +218,7 @@ struct BicgState {
     double rho[R], rho_new[R], alpha[R], omega[R], bb[R], rr[R], tol2[R];
     int iter[R], done[R], status[R];
     int all_done, max_iters;
+    unsigned int team[2];  // as PcgState::team
 };
 
 // zp[k][i] = (z_i, p_i): the preconditioned residual and the search

@@ -2,6 +2,7 @@
 #include "krylov_team.cuh"
 
 #include <algorithm>
+#include <cstdlib>
 
 #include <cooperative_groups.h>
 
@@ -24,6 +25,24 @@ constexpr int team_threads = RPT == 1 ? TEAM_R1 : CLUSTER ? 512 : 1024;
 constexpr int TEAM_CLUSTER = 16;      // blocks of the largest cluster
 constexpr unsigned TEAM_POLLS = 1u << 20;  // bound of a grid barrier's wait (about a second)
 
+// Bound of the waits; MC_TEAM_WAIT_POLLS lowers it (to make them run out).
+unsigned team_polls()
+{
+    const char *v = std::getenv("MC_TEAM_WAIT_POLLS");
+    if (v && *v) {
+        const long n = std::strtol(v, nullptr, 10);
+        if (n >= 0 && n < (long)TEAM_POLLS) return (unsigned)n;
+    }
+    return TEAM_POLLS;
+}
+
+// Device memory of the grid form's barrier, as a kernel gets it.
+struct TeamMem {
+    unsigned int *words;  // arrivals; a block's wait ran out (both zero at the launch)
+    double *partials;
+    unsigned int polls;
+};
+
 // The blocks of the team and their sum-and-barrier.  Every thread of every
 // block calls sums() the same number of times; the totals are the same bits in
 // every thread, so all blocks take the same branches.
@@ -37,7 +56,9 @@ struct Team {
     double *tot;                      // [4] shared: totals, tot[3] != 0: a wait ran out
 
     // Totals of v over the team, and a barrier: what any thread stored before
-    // is visible to loads after.  False when a wait ran out.
+    // is visible to loads after.  False when this block's wait ran out, which
+    // m.words[1] then tells the host: the other blocks need not notice (the
+    // last one to arrive waits for none).
     template <int K>
     __device__ __forceinline__ bool sums(double (&v)[K])
     {
@@ -74,12 +95,13 @@ struct Team {
                 if (lane == 0) part[(size_t)k * size + rank] = b;
             }
             if (lane == 0) {
-                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(m.arrive) : "memory");
+                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(m.words) : "memory");
                 unsigned seen, polls = 0;
                 do {
-                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(m.arrive) : "memory");
-                } while (seen < epoch * (unsigned)size && ++polls < TEAM_POLLS);
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(m.words) : "memory");
+                } while (seen < epoch * (unsigned)size && ++polls < m.polls);
                 tot[3] = seen < epoch * (unsigned)size ? 1.0 : 0.0;
+                if (seen < epoch * (unsigned)size) *(volatile unsigned int *)(m.words + 1) = 1u;
             }
             __syncwarp();
 #pragma unroll
@@ -160,10 +182,7 @@ __global__ void __launch_bounds__((team_threads<CLUSTER, RPT>), 1)
         a3[1] += r[e] * z[e];
         a3[2] += r[e] * r[e];
     }
-    if (!team.sums(a3)) {
-        if (t == 0) v.st->done = 1, v.st->status = KRYLOV_TIMEOUT;
-        return;
-    }
+    if (!team.sums(a3)) return;
     const double tol = fmax(rtol * sqrt(a3[0]), abs_floor), tol2 = tol * tol;
     double rz = a3[1], rz_old = 1.0, rr = a3[2];
     int iter = 0, status = KRYLOV_OK;
@@ -386,7 +405,7 @@ __global__ void __launch_bounds__((team_threads<CLUSTER, RPT>), 1)
         st->omega[0] = omega;
         st->iter[0] = iter;
         st->done[0] = 1;
-        st->status[0] = fine ? status : (int)KRYLOV_TIMEOUT;
+        st->status[0] = status;
         st->all_done = 1;
         st->max_iters = max_iters;
     }
@@ -429,7 +448,7 @@ TeamShape team_shape(int N)
 // Launch k on the team, or false (no error left behind) when the device does
 // not take the launch.
 template <typename... KArgs, typename... Args>
-bool team_launch(void (*k)(KArgs...), const TeamShape &sh, size_t smem, cudaStream_t s, const TeamMem &m,
+bool team_launch(void (*k)(KArgs...), const TeamShape &sh, size_t smem, cudaStream_t s, unsigned int *words,
                  Args &&...args)
 {
     bool ok = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
@@ -454,7 +473,8 @@ bool team_launch(void (*k)(KArgs...), const TeamShape &sh, size_t smem, cudaStre
         at[0].val.cooperative = 1;
         int fit = 0;
         ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, sh.threads, smem) == cudaSuccess && fit > 0;
-        ok = ok && cudaMemsetAsync(m.arrive, 0, sizeof(unsigned int), s) == cudaSuccess;
+        // (a cluster waits in hardware: its words stay zero, as the state's memory was made)
+        ok = ok && cudaMemsetAsync(words, 0, 2 * sizeof(unsigned int), s) == cudaSuccess;
     }
     ok = ok && cudaLaunchKernelEx(&cfg, k, static_cast<Args &&>(args)...) == cudaSuccess;
     if (!ok) cudaGetLastError();
@@ -464,25 +484,27 @@ bool team_launch(void (*k)(KArgs...), const TeamShape &sh, size_t smem, cudaStre
 } // namespace
 
 bool pcg_team(cudaStream_t s, const Ell &A, const PcgVectors &v, double rtol, double abs_floor, int max_iters,
-              int use_x0, const TeamMem &m)
+              int use_x0)
 {
     const TeamShape sh = team_shape(A.N);
     if (!sh.blocks) return false;
     const size_t smem = team_smem(sh.rows, 0);
     auto k = sh.rpt == 1 ? (sh.cluster ? k_pcg_team<true, 1> : k_pcg_team<false, 1>)
                          : (sh.cluster ? k_pcg_team<true, 2> : k_pcg_team<false, 2>);
-    return team_launch(k, sh, smem, s, m, A, v, rtol, abs_floor, max_iters, use_x0, sh.rows, m);
+    return team_launch(k, sh, smem, s, v.st->team, A, v, rtol, abs_floor, max_iters, use_x0, sh.rows,
+                       TeamMem{v.st->team, v.partials, team_polls()});
 }
 
 bool bicg_team(cudaStream_t s, const Ell &A, const double *b, double *x, double2 *rp, double *vv0, double *vv1,
-               BicgState<1> *st, double rtol, int max_iters, const TeamMem &m)
+               double *partials, BicgState<1> *st, double rtol, int max_iters)
 {
     const TeamShape sh = team_shape(A.N);
     if (!sh.blocks) return false;
     const size_t smem = team_smem(sh.rows, 2);
     auto k = sh.rpt == 1 ? (sh.cluster ? k_bicg_team<true, 1> : k_bicg_team<false, 1>)
                          : (sh.cluster ? k_bicg_team<true, 2> : k_bicg_team<false, 2>);
-    return team_launch(k, sh, smem, s, m, A, b, x, rp, vv0, vv1, st, rtol, max_iters, sh.rows, m);
+    return team_launch(k, sh, smem, s, st->team, A, b, x, rp, vv0, vv1, st, rtol, max_iters, sh.rows,
+                       TeamMem{st->team, partials, team_polls()});
 }
 
 } // namespace mcb

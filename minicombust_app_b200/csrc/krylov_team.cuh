@@ -19,23 +19,25 @@
 
 namespace mcb {
 
-// Device memory of the grid form's barrier; arrive must be zero at the launch.
-struct TeamMem {
-    unsigned int *arrive = nullptr;
-    double *partials = nullptr;  // [2][3][SMs]
-};
+// Status of a finished team solve: the grid form's waits are bounded, and a block
+// whose wait ran out has left without its rows' result whatever the others did.
+template <typename State>
+int team_status(const State &st, int status)
+{
+    return st.team[1] ? (int)KRYLOV_TIMEOUT : status;
+}
 
 // Jacobi-preconditioned CG (the method of k_pcg_init, k_pcg_iter1 and
 // k_pcg_iter2, with the mean-zero projections): v.st->mean set when project
 // (pcg_mean), v.x the initial guess when use_x0, else zero.  One launch leaves
-// the solution (mean removed) in v.x and the state in v.st.  False (nothing
-// launched) where no team holds N rows.
+// the solution (mean removed) in v.x and the state in v.st (team_status).  v.partials:
+// [2][3][SMs] at least.  False (nothing launched) where no team holds N rows.
 bool pcg_team(cudaStream_t s, const Ell &A, const PcgVectors &v, double rtol, double abs_floor, int max_iters,
-              int use_x0, const TeamMem &m);
+              int use_x0);
 
 // BiCGStab with one right-hand side (k_bicg_init, _1, _2, _3) from zero.
-// rp: [N] pairs, vv: two vectors [N].
+// rp: [N] pairs, vv: two vectors [N], partials as for pcg_team.
 bool bicg_team(cudaStream_t s, const Ell &A, const double *b, double *x, double2 *rp, double *vv0, double *vv1,
-               BicgState<1> *st, double rtol, int max_iters, const TeamMem &m);
+               double *partials, BicgState<1> *st, double rtol, int max_iters);
 
 } // namespace mcb

@@ -42,12 +42,11 @@ constexpr int kMaxBlocks = (kMaxRows + MCB_THREADS - 1) / MCB_THREADS;
 constexpr int kPartialsPerBlock = 8;
 static_assert(MCB_THREADS == 256, "scratch partitioning assumes 256-thread Krylov blocks");
 static_assert(kPartialsPerBlock >= 2, "BiCGStab with one right-hand side publishes 2 partials per block");
-constexpr size_t kStatusDoubles = 64;             // counter (first 8 bytes) + BicgState<1> + the team's barrier word
-constexpr size_t kArriveDouble = 48;              // where that word is
+constexpr size_t kStatusDoubles = 64;             // counter (first 8 bytes) + BicgState<1>
 constexpr size_t kScratchDoubles =
     (size_t)kVectors * kMaxRows + (size_t)kMaxBlocks * kPartialsPerBlock + kStatusDoubles;
 
-static_assert(sizeof(mcb::BicgState<1>) + 8 <= kArriveDouble * sizeof(double), "status block too small");
+static_assert(sizeof(mcb::BicgState<1>) + 8 <= kStatusDoubles * sizeof(double), "status block too small");
 
 static __device__ __align__(256) double g_scratch[kScratchDoubles];
 
@@ -108,13 +107,13 @@ extern "C" int mc_solve_bicgstab_noalloc(int n, const double *diag, const double
     mcb::BicgState<1> hs{};
     auto status_of = [&]() -> int {
         if (iterations) *iterations = hs.iter[0];
-        if (hs.status[0] == mcb::KRYLOV_NONFINITE) return MC_ERR_NONFINITE;
-        if (hs.status[0] == mcb::KRYLOV_TIMEOUT) return MC_ERR_TIMEOUT;
-        return hs.status[0] == mcb::KRYLOV_OK ? MC_OK : MC_ERR_NOT_CONVERGED;
+        const int status = mcb::team_status(hs, hs.status[0]);
+        if (status == mcb::KRYLOV_NONFINITE) return MC_ERR_NONFINITE;
+        if (status == mcb::KRYLOV_TIMEOUT) return MC_ERR_TIMEOUT;
+        return status == mcb::KRYLOV_OK ? MC_OK : MC_ERR_NOT_CONVERGED;
     };
     // the whole solve in one kernel: (r, p) pairs in the place of r and r0
-    const mcb::TeamMem team{(unsigned int *)(status + kArriveDouble), v.partials};
-    if (mcb::bicg_team(s, A, b, x, (double2 *)v.r, v.v[0], v.v[1], v.st, rtol, max_iters, team)) {
+    if (mcb::bicg_team(s, A, b, x, (double2 *)v.r, v.v[0], v.v[1], v.partials, v.st, rtol, max_iters)) {
         if (cudaMemcpyAsync(&hs, v.st, sizeof(hs), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MC_ERR_CUDA;
         if (cudaStreamSynchronize(s) != cudaSuccess) return MC_ERR_CUDA;
         return status_of();

@@ -12,6 +12,9 @@ differ by at most 2e-12 times the condition number (below 1e4 at these sizes)
 relative to the correction, itself a small part of the fields: 1e-9.
 """
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -69,3 +72,66 @@ def test_pcg_team_matches_amg(gpu, dims, reorder):
         s.close()
     for n, a in out[0].items():
         assert np.abs(a - out[1][n]).max() <= 1e-9 * np.abs(a).max(), n
+
+
+CHILD = r"""
+import ctypes, os, sys
+sys.path.insert(0, os.environ["MC_ROOT"])
+import numpy as np
+import torch
+from minicombust_app_b200 import flow
+from minicombust_app_b200.workload import noisy_fields
+L = flow.library()
+n = 40000
+idx = np.arange(n, dtype=np.int32)
+off, col = np.zeros((6, n)), np.tile(idx, (6, 1))
+off[0, 1:], col[0, 1:] = -1.0, idx[:-1]
+dev = [torch.from_numpy(a).cuda() for a in (np.full(n, 2.0), off, col, np.ones(n))]
+x = torch.zeros(n, dtype=torch.float64, device="cuda")
+def solve():
+    torch.cuda.synchronize()
+    return L.mc_solve_bicgstab_noalloc(n, *(t.data_ptr() for t in dev), x.data_ptr(), 1e-10, 200, None, None)
+s = flow.FlowSolver(flow.Mesh.box(40, 30, 30, 0.2, 0.1, 0.1), params=flow.default_params(flow.MODE_SIMPLE, max_iters=49))
+s1 = flow.FlowSolver(flow.Mesh.box(40, 30, 30, 0.2, 0.1, 0.1), params=flow.default_params(flow.MODE_SIMPLE))
+for h in (s, s1):
+    for name, vals in noisy_fields(h.N, 5).items():
+        a = h.field(name)
+        a[:h.N] = vals
+        h.set_field(name, a)
+    h.stage("gradients")
+    h.stage("momentum")
+def stage(h, name):
+    try:
+        h.stage(name)
+    except flow.FlowError as e:
+        return e.status
+    return flow.MC_OK
+before = s1.field("P")
+os.environ["MC_TEAM_WAIT_POLLS"] = "0"
+for _ in range(3):
+    assert solve() == flow.MC_ERR_TIMEOUT
+assert stage(s1, "pressure") == flow.MC_ERR_TIMEOUT
+assert np.array_equal(before[:s1.N], s1.field("P")[:s1.N])
+assert stage(s, "temperature") == flow.MC_ERR_TIMEOUT  # 49 iterations: BiCGStab, not sweeps
+del os.environ["MC_TEAM_WAIT_POLLS"]
+for _ in range(2):
+    assert solve() == flow.MC_OK
+    want = np.zeros(n)
+    for k in range(60):  # x_i = (1 + x_{i-1}) / 2
+        want = (1.0 + np.concatenate([[0.0], want[:-1]])) / 2
+    assert np.abs(x.cpu().numpy() - want).max() <= 1e-8
+    assert stage(s1, "pressure") == flow.MC_OK
+    assert stage(s, "temperature") in (flow.MC_OK, flow.MC_ERR_NOT_CONVERGED)
+print("team timeout ok")
+"""
+
+
+def test_wait_that_runs_out_is_reported_and_recovers(gpu):
+    """With a bound of no polls a block that is not the last to arrive gives up at its
+    first barrier; the last one waits for none and cannot know.  (These sizes
+    take the grid form, so the per-kernel solvers did not run either.)"""
+    env = dict(os.environ, MC_ROOT=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    env.pop("MC_TEAM_WAIT_POLLS", None)
+    r = subprocess.run([sys.executable, "-c", CHILD], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert "team timeout ok" in r.stdout
