@@ -870,18 +870,25 @@ int solve_bicg(mc_flow *h, const Ell &A, const BicgVectors<R> &v, BicgState<R> *
 // sweep launched after the solve is done costs about a microsecond, reading
 // the state and launching again about fifteen).
 constexpr int SWEEP_BATCH = 6;
-constexpr int SWEEP_MAX = 40;
-// BiCGStab is kept where max_iters is below this: its iterations are what the
-// caller then bounds.
+// A solve is given up for BiCGStab when a system's residual stands still over a
+// batch; once the sweeps could have crossed the mesh, when at the reduction of
+// the last batch it would need more than SWEEP_PATIENCE further ones (90
+// BiCGStab iterations' bytes: one moves four times a sweep's); and after
+// SWEEP_MAX sweeps.  That is late on purpose.  Against and across the lines a
+// sweep carries a value one cell on, so the residual falls slowly (0.95 a sweep)
+// until the mesh is crossed, then fast; and flows whose sweeps are slow make
+// BiCGStab slower still.  Flows against, across and oblique to the lines, steps
+// of 1e-4 to 1, relaxation 0.7 to 1, 12,000 to 524,000 cells, to 1e-8: wherever
+// the sweeps got there they were the faster method, by 1.1 to 500 times
+// (524,000 cells, ms: 35 sweeps 1.0, 32 iterations 3.6; 95 sweeps 2.8, 176
+// iterations 20; 250 sweeps, at 0.93 each, 4.2, 333 iterations 16); nine of 99
+// stalled.
+constexpr int SWEEP_PATIENCE = 60;
+constexpr int SWEEP_MAX = 600;
+// In FP64, BiCGStab is kept where max_iters is below this: its iterations are
+// what the caller then bounds.
 constexpr int SWEEP_MIN_ITERS = 50;
 
-// The solve by FP64 x-line sweeps (krylov.cuh), x[j] the solutions and
-// `scratch` [R][N] the other iterate.  Returns MC_OK with *used set when every
-// system met ||b - A x|| <= u_rtol ||b||; *used = false when the splitting is
-// not the faster method here -- a sweep that does not halve the residual of an
-// open system (a BiCGStab iteration moves four times a sweep's bytes and takes
-// about a decade off), or a non-finite value -- and the caller runs BiCGStab
-// from zero.
 // With FP32 refinement the sweeps are used unless ir_line_steps asks for the
 // inner BiCGStab: in FP64 they move 448 bytes per row for the three momentum
 // systems, fewer than FP32 sweeps with an FP64 residual after each pair
@@ -892,6 +899,11 @@ bool sweeps_apply(const mc_flow *h)
     return h->line64.ex > 0 && h->prm.max_iters >= SWEEP_MIN_ITERS && (!h->bir_mem || h->prm.ir_line_steps > 0);
 }
 
+// The solve by FP64 x-line sweeps (krylov.cuh), x[j] the solutions and
+// `scratch` [R][N] the other iterate.  Returns MC_OK with *used set when every
+// system met ||b - A x|| <= u_rtol ||b||; *used = false when the sweeps stall
+// (SWEEP_PATIENCE) or meet a non-finite value, and the caller runs BiCGStab
+// from zero.
 template <int R>
 int solve_sweeps(mc_flow *h, const double *diag, const double *off, const double *b, double *const (&x)[R],
                  double *scratch, SweepState<R> *st, SweepState<R> *hs, int iters_out[R], bool *used)
@@ -910,7 +922,10 @@ int solve_sweeps(mc_flow *h, const double *diag, const double *off, const double
     v.partials = h->partials;
     v.counter = h->counter;
     v.st = st;
-    for (int k = 0; k < SWEEP_MAX;) {
+    const int limit = std::min(SWEEP_MAX, h->prm.max_iters);
+    const int across = L.ex + 2 * (int)std::sqrt((double)(h->N / L.ex));  // cells of a box's three edges, about
+    double before[R];                                                     // residual norms squared, a batch earlier
+    for (int k = 0; k < limit;) {
         for (int q = 0; q < SWEEP_BATCH; q++, k++)
             launch(h, R == 3 ? K_SWEEP3 : K_SWEEP1, [&] { line_sweep64<R>(h->stream, L, v, k, h->prm.u_rtol); });
         const int rc = check_launch(h);
@@ -920,8 +935,17 @@ int solve_sweeps(mc_flow *h, const double *diag, const double *off, const double
         flush_timing(h);
         if (hs->nonfinite) return MC_OK;
         if (hs->all_done) break;
-        for (int j = 0; j < R; j++)
-            if (!hs->done[j] && !(hs->rr[j] <= 0.25 * hs->rr_prev[j])) return MC_OK;
+        for (int j = 0; j < R; j++) {
+            if (k > SWEEP_BATCH && !hs->done[j]) {
+                const double r = hs->rr[j], was = before[j];
+                if (std::fabs(r - was) <= 1e-3 * was) return MC_OK;
+                // (negated: nothing is expected of a residual that grew or a tolerance of zero)
+                if (k >= across &&
+                    !(r < was && std::log(hs->tol2[j] / r) >= SWEEP_PATIENCE * std::log(r / was)))
+                    return MC_OK;
+            }
+            before[j] = hs->rr[j];
+        }
     }
     if (!hs->all_done) return MC_OK;
     if (hs->where == 1)

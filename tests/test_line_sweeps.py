@@ -1,8 +1,8 @@
 """The FP64 x-line sweeps (momentum, temperature and scalar solves on boxes
 whose cells run x-fastest) against the CPU oracle, whose solves are BiCGStab:
 line lengths at the edges of the 32-cell scan chunks, meshes of a few lines,
-handles that renumber their cells, and a flow across the lines with a long time
-step, where the splitting converges too slowly and BiCGStab takes over.
+handles that renumber their cells, and flows across the lines: slow sweeps, and
+with a long time step ones too slow to go on with, where BiCGStab takes over.
 
 Solves run to 1e-12 on both sides; fields agree to 1e-9 of their maximum, the
 parity gate of the other whole-pass tests (the transient term bounds the
@@ -19,22 +19,24 @@ pytestmark = pytest.mark.gpu
 BASE = {"U": 50.0, "V": 0.0, "W": 0.0, "P": 4000.0, "TEM": 1500.0}
 
 
-def run_both(dims, passes=2, base=BASE, **kw):
+def run_both(dims, passes=2, base=BASE, counts=None, **kw):
     lengths = (0.2, 0.1, 0.1)
-    p = flow.default_params(flow.MODE_SIMPLE, u_rtol=1e-12, p_rtol=1e-12, **kw)
+    p = flow.default_params(flow.MODE_SIMPLE, **{"u_rtol": 1e-12, "p_rtol": 1e-12, **kw})
     solver = flow.FlowSolver(flow.Mesh.box(*dims, *lengths), params=p)
     okw = {"u_rtol": 1e-12, "p_rtol": 1e-12}
-    if "delta" in kw:
-        okw["delta"] = kw["delta"]
+    okw.update({k: kw[k] for k in ("delta", "urf_momentum") if k in kw})
     orc = Oracle(oracle_mesh(*dims, *lengths), oracle_params(SIMPLE, scalars=p.transport_scalars, **okw))
     for name, vals in noisy_initial_fields(solver.N, base, 1).items():
         for s in (solver, orc):
             a = s.field(name)
             a[:solver.N] = vals
             s.set_field(name, a)
+    solver.set_timing(counts is not None)
     for _ in range(passes):
         solver.simple_iteration()
         orc.step()
+    if counts is not None:
+        counts.update({k: n for k, (_, n) in solver.kernel_times().items()})
     for name in BASE:
         a, b = solver.field(name), orc.field(name)
         assert np.abs(a - b).max() <= 1e-9 * np.abs(b).max(), (dims, name)
@@ -69,5 +71,27 @@ def test_scalars_by_sweeps_match_oracle(gpu):
     run_both((33, 6, 5), transport_scalars=1)
 
 
-def test_cross_flow_falls_back_to_bicgstab(gpu):
+@pytest.mark.parametrize("precision", [flow.PRECISION_FP64, flow.PRECISION_FP32_REFINED], ids=["fp64", "refined"])
+@pytest.mark.parametrize("urf", [0.7, 1.0])
+def test_slow_sweeps_are_kept(gpu, precision, urf):
+    """A sweep takes off less than half of the residual here, the first ones a tenth,
+    and some 60 sweeps still cost a fraction of BiCGStab's iterations."""
+    n = {}
+    st = run_both((24, 32, 16), passes=1, base={**BASE, "U": 1.0, "V": 80.0}, delta=1e-3, counts=n,
+                  pressure_solver=flow.PSOLVER_PCG_AMG, precision=precision, urf_momentum=urf)
+    assert max(st.momentum_iters) > 20 and st.temperature_iters > 20
+    assert n["line_sweep3_64"] >= max(st.momentum_iters) and n["line_sweep1_64"] >= st.temperature_iters
+    assert all(n[k] == 0 for k in n if k.startswith("bicg"))
+
+
+def test_long_step_cross_flow_matches_oracle(gpu):
     run_both((12, 24, 6), passes=1, base={**BASE, "U": 1.0, "V": 80.0}, delta=1e-2)
+
+
+def test_stalled_sweeps_fall_back_to_bicgstab(gpu):
+    """The sweeps' true residual cannot reach 1e-17 ||b||, the recursive one of
+    BiCGStab can: the stall is seen within three batches."""
+    n = {}
+    run_both((12, 24, 6), passes=1, counts=n, u_rtol=1e-17)
+    assert n["bicg3_init"] == 1 and n["bicg1_team"] == 1
+    assert 0 < n["line_sweep3_64"] <= 18 and 0 < n["line_sweep1_64"] <= 18
