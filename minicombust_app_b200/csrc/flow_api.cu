@@ -886,7 +886,8 @@ constexpr int SWEEP_BATCH = 6;
 constexpr int SWEEP_PATIENCE = 60;
 constexpr int SWEEP_MAX = 600;
 // In FP64, BiCGStab is kept where max_iters is below this: its iterations are
-// what the caller then bounds.
+// what the caller then bounds (with FP32 refinement max_iters bounds the inner
+// solves alone).
 constexpr int SWEEP_MIN_ITERS = 50;
 
 // With FP32 refinement the sweeps are used unless ir_line_steps asks for the
@@ -896,7 +897,8 @@ constexpr int SWEEP_MIN_ITERS = 50;
 // assembly 0.02 less without the FP32 rows), and their errors are 100 times smaller.
 bool sweeps_apply(const mc_flow *h)
 {
-    return h->line64.ex > 0 && h->prm.max_iters >= SWEEP_MIN_ITERS && (!h->bir_mem || h->prm.ir_line_steps > 0);
+    if (h->line64.ex == 0) return false;
+    return h->bir_mem ? h->prm.ir_line_steps > 0 : h->prm.max_iters >= SWEEP_MIN_ITERS;
 }
 
 // The solve by FP64 x-line sweeps (krylov.cuh), x[j] the solutions and
@@ -922,7 +924,7 @@ int solve_sweeps(mc_flow *h, const double *diag, const double *off, const double
     v.partials = h->partials;
     v.counter = h->counter;
     v.st = st;
-    const int limit = std::min(SWEEP_MAX, h->prm.max_iters);
+    const int limit = h->bir_mem ? SWEEP_MAX : std::min(SWEEP_MAX, h->prm.max_iters);
     const int across = L.ex + 2 * (int)std::sqrt((double)(h->N / L.ex));  // cells of a box's three edges, about
     double before[R];                                                     // residual norms squared, a batch earlier
     for (int k = 0; k < limit;) {

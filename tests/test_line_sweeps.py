@@ -84,6 +84,16 @@ def test_slow_sweeps_are_kept(gpu, precision, urf):
     assert all(n[k] == 0 for k in n if k.startswith("bicg"))
 
 
+def test_refined_sweeps_whatever_max_iters(gpu):
+    """With FP32 refinement max_iters bounds the inner solves, not the sweeps."""
+    n = {}
+    st = run_both((24, 12, 10), counts=n, max_iters=20, pressure_solver=flow.PSOLVER_PCG_AMG,
+                  precision=flow.PRECISION_FP32_REFINED)
+    assert n["line_sweep3_64"] > 0 and n["line_sweep1_64"] > 0
+    assert all(n[k] == 0 for k in n if k.startswith("bicg"))
+    assert 1 <= max(st.momentum_iters) <= 12 and 1 <= st.temperature_iters <= 12
+
+
 def test_long_step_cross_flow_matches_oracle(gpu):
     run_both((12, 24, 6), passes=1, base={**BASE, "U": 1.0, "V": 80.0}, delta=1e-2)
 
