@@ -92,6 +92,7 @@ struct mc_gnn {
     int t = 0;
     char *work_mem = nullptr;
     size_t work_bytes = 0;
+    int work_asked = 0;  // samples the work area was asked for (it may hold fewer)
     GnnWork work;
     double *h_loss = nullptr;  // pinned [GNN_MAX_BATCH][2]
 };
@@ -120,21 +121,29 @@ int cuda_status(cudaError_t e) { return e == cudaSuccess ? MC_OK : (e == cudaErr
         if (rc_) return rc_;                   \
     } while (0)
 
-// Work area for inference (samples 0) or training of `samples` at a time; a
-// training area also serves inference on the same graph size.
+// Work area for inference (samples 0) or training of `samples` at a time, or of
+// fewer where their memory cannot be had; a training area also serves
+// inference on the same graph size.
 int ensure_work(mc_gnn *net, int n, int samples)
 {
-    const size_t need = gnn_work_bytes(n, samples);
-    if (net->work_mem && net->work.n == n && net->work.samples >= samples) return MC_OK;
+    if (net->work_mem && net->work.n == n && net->work_asked >= samples) return MC_OK;
     if (net->work_mem) {
         cudaStreamSynchronize(net->stream);
         cudaFree(net->work_mem);
         net->work_mem = nullptr;
     }
-    GNN_TRY(cudaMalloc((void **)&net->work_mem, need));
-    GNN_TRY(cudaMemsetAsync(net->work_mem, 0, need, net->stream));
-    net->work_bytes = need;
-    gnn_work_carve(net->work, net->work_mem, n, samples);
+    int q = samples;
+    for (;; q /= 2) {
+        net->work_bytes = gnn_work_bytes(n, q);
+        const cudaError_t e = cudaMalloc((void **)&net->work_mem, net->work_bytes);
+        if (e == cudaSuccess) break;
+        net->work_mem = nullptr;
+        cudaGetLastError();  // reported here, or by a smaller area taken instead
+        if (e != cudaErrorMemoryAllocation || q <= 1) return cuda_status(e);
+    }
+    GNN_TRY(cudaMemsetAsync(net->work_mem, 0, net->work_bytes, net->stream));
+    gnn_work_carve(net->work, net->work_mem, n, q);
+    net->work_asked = samples;
     return MC_OK;
 }
 
