@@ -2573,7 +2573,9 @@ int mc_flow_create(const mc_mesh_view *mesh, const mc_flow_params *params, mc_fl
             m.xc = h->xc; m.yc = h->yc; m.zc = h->zc;
             m.vol = h->vol; m.rho = h->rho;
             m.outlet_faces = h->outlet_faces;
-            // (the boundary balance's memory takes the flag: nothing has run yet)
+            // (the boundary balance's memory takes the flag: nothing has run yet; the
+            // centres were copied on the default stream, which h->stream does not wait for)
+            cudaStreamSynchronize(cudaStreamLegacy);
             int *flag = reinterpret_cast<int *>(h->balance), off = 1;
             launch_face_offsets(h->stream, krylov_grid(h->F), h->N, m, flag);
             if (cudaMemcpyAsync(&off, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||

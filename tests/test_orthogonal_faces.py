@@ -55,3 +55,21 @@ def test_displaced_centres_take_the_general_form(gpu):
         assert box.last_stats.pressure_iters_total == box.last_stats.pressure_iters_first
         s.close()
         box.close()
+
+
+@pytest.mark.parametrize("cell", [0, -1], ids=["first", "last"])
+def test_one_displaced_centre_is_found(gpu, cell):
+    """The check at creation sees every cell, the last ones uploaded too."""
+    mesh = flow.Mesh.box(96, 40, 40, 0.2, 0.1, 0.1)
+    mesh.cell_centers[cell] += 2e-4
+    for _ in range(3):
+        s = flow.FlowSolver(mesh, params=flow.default_params(flow.MODE_SIMPLE, pressure_solver=flow.PSOLVER_PCG_AMG,
+                                                             p_rtol=1e-12))
+        for name, vals in noisy_initial_fields(s.N, {"U": 50.0, "V": 0.0, "W": 0.0, "P": 4000.0, "TEM": 1500.0},
+                                               3).items():
+            a = s.field(name)
+            a[:s.N] = vals
+            s.set_field(name, a)
+        s.simple_iteration()
+        assert s.last_stats.pressure_iters_total > s.last_stats.pressure_iters_first
+        s.close()
