@@ -254,6 +254,8 @@ int mc_gnn_graph_create(mc_gnn *net, const mc_mesh_view *mesh, mc_gnn_graph **ou
     if (!rc) rc = cuda_status(cudaMemcpy(gr->mem + cb, edge.data(), eb, cudaMemcpyHostToDevice));
     if (!rc) rc = cuda_status(cudaMemcpy(gr->mem + cb + eb, vhat.data(), vb, cudaMemcpyHostToDevice));
     if (!rc && mb) rc = cuda_status(cudaMemcpy(gr->mem + cb + eb + vb, mask.data(), mb, cudaMemcpyHostToDevice));
+    // the copies are made on the default stream, which no network's stream waits for
+    if (!rc) rc = cuda_status(cudaStreamSynchronize(cudaStreamLegacy));
     if (rc) {
         mc_gnn_graph_destroy(gr);
         return rc;

@@ -167,3 +167,20 @@ def test_tensor_core_layer_matches_mma_layer_on_many_tiles(gpu, monkeypatch):
     # outputs differ only where a BF16 rounding falls the other way
     assert rel(ys["umma"], ys["mma"]) <= 1e-2
     assert np.mean(np.abs(ys["umma"] - ys["mma"]) <= 1e-2 * np.abs(ys["mma"]).max()) > 0.99
+
+
+def test_first_prediction_on_a_graph(gpu):
+    """A graph's arrays are on the device when it has been created: the first
+    prediction on it is the second one's."""
+    import torch
+    mesh = flow.Mesh.box(96, 48, 48, 0.2, 0.1, 0.1)
+    net = gnn.GuessNet(seed=1)
+    rhs = torch.randn(mesh.n_cells, device="cuda")
+    diag = torch.rand(mesh.n_cells, device="cuda") + 1.0
+    torch.cuda.synchronize()
+    y = [torch.empty(mesh.n_cells, device="cuda") for _ in range(2)]
+    for _ in range(3):
+        gr = net.graph(mesh)
+        for k in range(2):
+            net.predict(gr, rhs, diag, y=y[k])
+        assert torch.equal(*y)
