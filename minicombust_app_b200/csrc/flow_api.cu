@@ -286,6 +286,23 @@ void launch(mc_flow *h, int kid, Fn &&fn)
     h->launches++;
 }
 
+// The same for a launch that may be declined: fn says whether it was made, and
+// one that was not is not counted or timed.
+template <typename Fn>
+bool launch_if(mc_flow *h, int kid, Fn &&fn)
+{
+    bool made = false;
+    launch(h, kid, [&] { made = fn(); });
+    if (!made) {
+        h->launches--;
+        if (h->timing.on) {
+            h->timing.used--;
+            h->timing.ids.pop_back();
+        }
+    }
+    return made;
+}
+
 void flush_timing(mc_flow *h)
 {
     Timing &t = h->timing;
@@ -619,11 +636,9 @@ int solve_pressure(mc_flow *h, double abs_floor, int *iters, double *relres, dou
     if (const int rl = launch_deferred_inverse(h)) return rl;
     if (!amg) {
         // small systems: the whole solve in one kernel
-        bool team = false;
-        launch(h, K_PCG_TEAM, [&] {
-            team = pcg_team(h->stream, A, v, h->prm.p_rtol, abs_floor, h->prm.max_iters, use_x0);
-        });
-        if (team) {
+        if (launch_if(h, K_PCG_TEAM, [&] {
+                return pcg_team(h->stream, A, v, h->prm.p_rtol, abs_floor, h->prm.max_iters, use_x0);
+            })) {
             CUDA_TRY(h, cudaMemcpyAsync(h->h_pcg, v.st, sizeof(PcgState), cudaMemcpyDeviceToHost, h->stream));
             CUDA_TRY(h, cudaStreamSynchronize(h->stream));
             flush_timing(h);
@@ -633,7 +648,6 @@ int solve_pressure(mc_flow *h, double abs_floor, int *iters, double *relres, dou
             *relres = s.bb > 0 ? std::sqrt(s.rr / s.bb) : 0.0;
             return krylov_status_to_mc(team_status(s, s.status));
         }
-        h->launches--;
     }
     if (amg) {
         launch(h, K_PCG_INIT_AMG,
@@ -818,19 +832,16 @@ int solve_bicg(mc_flow *h, const Ell &A, const BicgVectors<R> &v, BicgState<R> *
                cudaGraphExec_t *loop, int kid_init, int kid1, int iters_out[R])
 {
     if constexpr (R == 1) {  // small systems: the whole solve in one kernel
-        bool team = false;
-        launch(h, K_BICG1_TEAM, [&] {
-            team = bicg_team(h->stream, A, v.b, v.x[0], h->pv.zp[0], v.v[0], v.v[1], v.partials, v.st,
-                             h->prm.u_rtol, h->prm.max_iters);
-        });
-        if (team) {
+        if (launch_if(h, K_BICG1_TEAM, [&] {
+                return bicg_team(h->stream, A, v.b, v.x[0], h->pv.zp[0], v.v[0], v.v[1], v.partials, v.st,
+                                 h->prm.u_rtol, h->prm.max_iters);
+            })) {
             CUDA_TRY(h, cudaMemcpyAsync(hs, v.st, sizeof(BicgState<R>), cudaMemcpyDeviceToHost, h->stream));
             CUDA_TRY(h, cudaStreamSynchronize(h->stream));
             flush_timing(h);
             iters_out[0] = hs->iter[0];
             return krylov_status_to_mc(team_status(*hs, hs->status[0]));
         }
-        h->launches--;
     }
     launch(h, kid_init, [&] { bicg_init<R>(h->stream, A, v, h->prm.u_rtol, h->prm.max_iters); });
     int rc = check_launch(h);

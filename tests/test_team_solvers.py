@@ -74,6 +74,22 @@ def test_pcg_team_matches_amg(gpu, dims, reorder):
         assert np.abs(a - out[1][n]).max() <= 1e-9 * np.abs(a).max(), n
 
 
+@pytest.mark.parametrize("dims,team", [((17, 11, 11), True), ((80, 44, 43), True), ((80, 60, 63), True),
+                                       ((80, 64, 60), False)])
+def test_kernel_counts_name_the_solver_that_ran(gpu, dims, team):
+    """A cluster, the grid up to 2,048 rows per SM, the per-kernel solver above."""
+    s = flow.FlowSolver(flow.Mesh.box(*dims, 0.2, 0.1, 0.1), params=flow.default_params(flow.MODE_SIMPLE))
+    for name, vals in noisy_fields(s.N, 5).items():
+        a = s.field(name)
+        a[:s.N] = vals
+        s.set_field(name, a)
+    s.set_timing(True)
+    s.simple_iteration()
+    n = {k: c for k, (_, c) in s.kernel_times().items()}
+    assert (n["pcg_team"] > 0) == team and (n["pcg_iter1_spmv"] > 0) == (not team)
+    s.close()
+
+
 CHILD = r"""
 import ctypes, os, sys
 sys.path.insert(0, os.environ["MC_ROOT"])
