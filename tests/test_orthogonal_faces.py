@@ -32,29 +32,36 @@ def test_box_matches_oracle(gpu, psolver, reorder):
         assert np.abs(a - b).max() <= 1e-9 * np.abs(b).max(), name
 
 
-def test_displaced_centres_take_the_general_form(gpu):
-    """Displaced centres make the flux correction non-zero, so a second
-    corrector has a right-hand side; the fluxes still balance to the solve's tolerance."""
-    mesh = flow.Mesh.box(12, 8, 8, 0.2, 0.1, 0.1)
-    rng = np.random.default_rng(0)
-    mesh.cell_centers += rng.uniform(-1, 1, mesh.cell_centers.shape) * 5e-4
-    for psolver in (flow.PSOLVER_PCG_JACOBI, flow.PSOLVER_PCG_AMG):
-        s = flow.FlowSolver(mesh, params=flow.default_params(flow.MODE_SIMPLE, pressure_solver=psolver, u_rtol=1e-12,
-                                                             p_rtol=1e-12))
-        box = flow.FlowSolver(flow.Mesh.box(12, 8, 8, 0.2, 0.1, 0.1),
-                              params=flow.default_params(flow.MODE_SIMPLE, pressure_solver=psolver, u_rtol=1e-12,
-                                                         p_rtol=1e-12))
-        for h in (s, box):
-            for name, vals in noisy_initial_fields(h.N, {"U": 50.0, "V": 0.0, "W": 0.0, "P": 4000.0, "TEM": 1500.0},
-                                                   3).items():
+@pytest.mark.parametrize("psolver", [flow.PSOLVER_PCG_JACOBI, flow.PSOLVER_PCG_AMG], ids=["jacobi", "amg"])
+@pytest.mark.parametrize("reorder", [flow.REORDER_NONE, flow.REORDER_RCM], ids=["natural", "rcm"])
+def test_displaced_centres_match_oracle(gpu, psolver, reorder):
+    """Displaced centres make the flux correction non-zero, so a second corrector
+    has a right-hand side: fields against the oracle, and the box, whose
+    second corrector has none, beside it."""
+    dims, lengths = (12, 8, 8), (0.2, 0.1, 0.1)
+    shift = np.random.default_rng(0).uniform(-1, 1, (12 * 8 * 8, 3)) * 5e-4
+    for displaced in (True, False):
+        mesh, om = flow.Mesh.box(*dims, *lengths), oracle_mesh(*dims, *lengths)
+        if displaced:
+            mesh.cell_centers += shift
+            om.cell_centers += shift
+        s = flow.FlowSolver(mesh, params=flow.default_params(flow.MODE_SIMPLE, pressure_solver=psolver, reorder=reorder,
+                                                             u_rtol=1e-13, p_rtol=1e-13))
+        o = Oracle(om, oracle_params(SIMPLE, u_rtol=1e-13, p_rtol=1e-13))
+        for name, vals in noisy_initial_fields(s.N, {"U": 50.0, "V": 0.0, "W": 0.0, "P": 4000.0, "TEM": 1500.0},
+                                               3).items():
+            for h in (s, o):
                 a = h.field(name)
-                a[:h.N] = vals
+                a[:s.N] = vals
                 h.set_field(name, a)
-            h.simple_iteration()
-        assert s.last_stats.pressure_iters_total > s.last_stats.pressure_iters_first
-        assert box.last_stats.pressure_iters_total == box.last_stats.pressure_iters_first
+        for _ in range(3):
+            s.simple_iteration()
+            o.step()
+            assert (s.last_stats.pressure_iters_total > s.last_stats.pressure_iters_first) == displaced
+        for name in ("U", "V", "W", "P", "TEM"):
+            a, b = s.field(name), o.field(name)
+            assert np.abs(a - b).max() <= 1e-9 * np.abs(b).max(), (displaced, name)
         s.close()
-        box.close()
 
 
 @pytest.mark.parametrize("cell", [0, -1], ids=["first", "last"])

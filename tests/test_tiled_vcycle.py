@@ -35,13 +35,14 @@ def run(dims, tiles, **kw):
         a = s.field(name)
         a[:s.N] = vals
         s.set_field(name, a)
-    its = []
+    its, before = [], s.launch_count()
     for _ in range(2):
         s.simple_iteration()
         its.append(s.last_stats.as_dict()["pressure_iters_total"])
+    launches = s.launch_count() - before
     fields = {n: s.field(n) for n in FIELDS}
     s.close()
-    return fields, its
+    return fields, its, launches
 
 
 @pytest.mark.parametrize("dims", [(26, 10, 8), (27, 11, 7), (52, 20, 9), (53, 21, 33), (25, 9, 31), (2, 30, 40),
@@ -49,18 +50,23 @@ def run(dims, tiles, **kw):
 @pytest.mark.parametrize("fp32", [False, True], ids=["fp64", "fp32"])
 def test_tiles_match_sweeps(gpu, dims, fp32):
     kw = dict(precision=flow.PRECISION_FP32_REFINED) if fp32 else {}
-    tiles, its_t = run(dims, "2", **kw)
-    sweeps, its_s = run(dims, "0", **kw)
+    tiles, its_t, n_t = run(dims, "2", **kw)
+    sweeps, its_s, n_s = run(dims, "0", **kw)
     assert its_t == its_s
+    # two kernels a level instead of six (FP32, paired sweeps) or eight; a
+    # small box may have no level above the single-block ones
+    assert n_t <= n_s and (n_t < n_s or np.prod(dims) < 8192)
     for n in FIELDS:
         rel = np.abs(tiles[n] - sweeps[n]).max() / np.abs(sweeps[n]).max()
         assert rel <= (1e-6 if fp32 else 1e-9), (n, rel)
 
 
 def test_rule_takes_tiles_at_a_large_box(gpu):
-    """At 256 x 128 x 128 the default rule tiles levels 0 and 1."""
-    rule, its_r = run((256, 128, 128), "1")
-    sweeps, its_s = run((256, 128, 128), "0")
+    """At 256 x 128 x 128 the default rule tiles levels 0 and 1: two kernels instead
+    of eight on each, in every V-cycle (one per iteration and one before the first)."""
+    rule, its_r, n_r = run((256, 128, 128), "1")
+    sweeps, its_s, n_s = run((256, 128, 128), "0")
     assert its_r == its_s
+    assert n_s - n_r >= sum(2 * 6 * (n + 1) for n in its_r)
     for n in FIELDS:
         assert np.abs(rule[n] - sweeps[n]).max() <= 1e-9 * np.abs(sweeps[n]).max(), n
