@@ -790,16 +790,20 @@ static TilePlan tile_plan(const int box[3])
 }
 
 // The tile kernels pay where their steps, overlap and idle blocks included, are
-// few per row.  V-cycles by sweeps and with tiles at six box sizes, FP64: 2.44
-// cell steps per row 321 -> 261 us (256 x 128 x 128), 2.57 249 -> 227 (128^3),
-// 3.03 234 -> 228 (320 x 64 x 100), 3.32 84 -> 76 (128 x 64 x 64), 3.44 118 ->
-// 118 (160 x 80 x 80), above that slower.  FP32 sweeps stream half the bytes:
-// 2.57 231 -> 188, 2.82 151 -> 153, 3.03 150 -> 160.
+// few per row.  Untimed passes of 6 pressure iterations by sweeps and with tiles,
+// FP64, by cell steps per row of level 0: 2.44 7.21 -> 6.90 ms (256 x 128 x 128),
+// 2.78 4.53 -> 4.44, 2.79 5.28 -> 5.14 and 4.16 -> 4.09, 2.85 2.85 -> 2.83; from
+// 3.02 to 3.25 ten boxes of 0.95 M to 2.3 M cells 0.2 % faster to 1.8 % slower.
+// Boxes of 0.5 M to 0.6 M cells gain the launches too: 3.09 1.71 -> 1.68, 3.11
+// 1.58 -> 1.56, 3.32 1.45 -> 1.44 (128 x 64 x 64, level 1 of the first).  FP32
+// sweeps stream half the bytes: 2.54 46.4 -> 45.4 (156 iterations), 2.57 6.57 ->
+// 6.23, 2.82 to 3.04 no gain.
 template <typename T>
 bool amg_tile_fits(const int box[3], int sweeps, int form)
 {
     if (form == 0 || sweeps != 3 || box[0] == 0) return false;
-    const double rows = (double)box[0] * box[1] * box[2], waste = sizeof(T) == 8 ? 3.35 : 2.7;
+    const double rows = (double)box[0] * box[1] * box[2];
+    const double waste = sizeof(T) == 4 ? 2.7 : rows <= 650000.0 ? 3.35 : 2.9;
     const TilePlan p = tile_plan<T>(box);
     // one partial sum per block, of the 24 per kernel grid block the solvers have
     if (p.blocks > 24L * krylov_grid((int)rows)) return false;

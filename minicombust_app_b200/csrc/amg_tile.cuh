@@ -14,10 +14,11 @@
 // these re-reads come from L2.  Values of the own column stay in registers, a
 // plane of each iterate in shared memory for the x and y neighbours; planes are
 // copied to shared memory five steps ahead (cp.async).  A step is bound by the
-// chain through shared memory and FP64 arithmetic, 0.65 us a plane at 16 warps:
-// FP64 V-cycles at 2 x 128^3 take 261 us, 321 by sweeps.  (Loading what only the
-// own column reads into registers two steps ahead: 305 us; the reciprocals a
-// plane ahead and split sums: 272.)
+// chain through shared memory and FP64 arithmetic, 0.65 us a plane at 16 warps: a
+// plain pass at 2 x 128^3, with six V-cycles that find work, takes 6.90 ms, 7.21
+// by sweeps.  (V-cycle time of an event-timed pass, ten launches: 2.64 ms; with
+// what only the own column reads loaded into registers two steps ahead 3.05,
+// with the reciprocals a plane ahead and split sums 2.72, by sweeps 3.23.)
 #pragma once
 
 #include <type_traits>

@@ -70,3 +70,12 @@ def test_rule_takes_tiles_at_a_large_box(gpu):
     assert n_s - n_r >= sum(2 * 6 * (n + 1) for n in its_r)
     for n in FIELDS:
         assert np.abs(rule[n] - sweeps[n]).max() <= 1e-9 * np.abs(sweeps[n]).max(), n
+
+
+@pytest.mark.parametrize("dims,tiled", [((128, 64, 64), True), ((80, 116, 141), False), ((200, 101, 97), False)])
+def test_rule_by_steps_per_row_and_size(gpu, dims, tiled):
+    """FP64: up to 2.9 cell steps per row, up to 3.35 below 650,000 cells (here 3.32,
+    3.19 and 3.13, the last two slower with tiles)."""
+    _, its, n_rule = run(dims, "1")
+    _, _, n_sweeps = run(dims, "0")
+    assert (n_sweeps - n_rule >= sum(6 * (n + 1) for n in its)) if tiled else n_rule == n_sweeps
