@@ -1311,10 +1311,9 @@ __global__ void __launch_bounds__(32 * R * sweep_lines<R>, sweep_blocks<R>)
             if (FIRST) {
                 if (on) sum += s * s;
             } else {
+                // every load before the shuffles, which wait for x0 and hold back what follows
                 const double x0 = xin[i];
-                double xm = __shfl_up_sync(0xffffffffu, x0, 1);
-                if (lane == 0) xm = xlast;
-                xlast = __shfl_sync(0xffffffffu, x0, 31);
+                double xm;
                 if (FORM == LINE_PERM) {
                     double o[6], xc[6];
 #pragma unroll
@@ -1322,6 +1321,7 @@ __global__ void __launch_bounds__(32 * R * sweep_lines<R>, sweep_blocks<R>)
                         o[k] = L.off[(size_t)k * N + i];
                         xc[k] = xin[L.col[(size_t)k * N + i]];
                     }
+                    xm = __shfl_up_sync(0xffffffffu, x0, 1);
 #pragma unroll
                     for (int k = 0; k < 6; k++) {
                         if (((cw >> (3 * k)) & 7u) == (unsigned)L.xm)
@@ -1340,11 +1340,14 @@ __global__ void __launch_bounds__(32 * R * sweep_lines<R>, sweep_blocks<R>)
                         xy[u] = xin[min(max(i + L.yzoff[u], 0), N - 1)];
                     }
                     double xp = __shfl_down_sync(0xffffffffu, x0, 1);
+                    xm = __shfl_up_sync(0xffffffffu, x0, 1);
                     if (lane == 31) xp = xe;
                     if (c + 1 < ex) s -= op * xp;
 #pragma unroll
                     for (int u = 0; u < 4; u++) s -= o[u] * xy[u];
                 }
+                if (lane == 0) xm = xlast;
+                xlast = __shfl_sync(0xffffffffu, x0, 31);
                 double res = s - d * x0;
                 if (c > 0) res -= a * xm;
                 if (on) sum += res * res;
