@@ -10,7 +10,7 @@ T0 1500 K; initial u, v, w, p, T = inlet state + seeded uniform noise +-1%;
 cells, amplitude 1e-3 of the cell inflow); the corrected SIMPLE pass
 (MC_MODE_SIMPLE), momentum URF 0.7, pressure URF 0.3, pressure PCG with the
 aggregation-AMG V-cycle (or Jacobi, --psolver jacobi) to rtol 1e-8,
-momentum/temperature BiCGStab to rtol 1e-8.  Synthetic data (the
+momentum/temperature by FP64 line sweeps to rtol 1e-8.  Synthetic data (the
 reference has no dataset); the working set (about 4.5 GB) is far larger than
 L2, so consecutive iterations stream from HBM.
 
@@ -145,9 +145,49 @@ class ClockSampler:
 
 # ------------------------------------------------------------- roofline
 
+def vcycle_tiled(box, fp32, sms):
+    """Whether a box level's halves of the V-cycle run as tile kernels (amg_tile_fits:
+    tiles of 26 x 10 own cells on 32 x 16 threads, a block per SM, two in FP32)."""
+    resident, cols = sms * (2 if fp32 else 1), -(-box[0] // 26) * -(-box[1] // 10)
+    steps = []
+    for c in range(1, max(1, box[2] // 4) + 1):
+        zc = (-(-box[2] // c) + 1) & ~1
+        steps.append(-(-cols * -(-box[2] // zc) // resident) * (zc + 7))
+    rows = box[0] * box[1] * box[2]
+    return min(steps) * resident * 512 <= (2.7 if fp32 else 3.35 if rows <= 650000 else 2.9) * rows
+
+
+def vcycle_bytes(box, fp32, sms, natural):
+    """One V-cycle: per level, tile kernels read each array once per half (right-hand
+    side, diagonal, three couplings, going up the iterate; an eighth of a value
+    for the coarse level; the iterate or result written): 106 bytes per row in
+    FP64, 53 in FP32.  Levels by sweeps: level 0 in FP64 (half form, 32 bytes of
+    matrix) first sweep 24, sweeps 4 x 56, restriction 53, prolongation 21, last
+    sweep 56 = 378, in FP32 (couplings in FP16) 168; the coarse levels 528 and
+    241.  The single-block levels of 1,024 rows and below are not counted."""
+    total, box, level0 = 0, list(box), True
+    while box[0] * box[1] * box[2] > 1024:
+        if natural and min(box) >= 2 and vcycle_tiled(box, fp32, sms):
+            row = 53 if fp32 else 106
+        else:
+            row = (168 if fp32 else 378) if level0 else (241 if fp32 else 528)
+        total += row * box[0] * box[1] * box[2]
+        box, level0 = [(x + 1) // 2 for x in box], False
+    return total
+
+
+def sweep_bytes(systems, N, sweeps):
+    """Mean over the sweeps of a line-sweep solve: the first reads diagonal, -x
+    coupling and right-hand sides and writes the iterates; the later ones read
+    the whole row, right-hand sides and iterates."""
+    return ((16 + 16 * systems) + (56 + 24 * systems) * (sweeps - 1)) / sweeps * N
+
+
 def kernel_bytes(name, N, F, nnz_off):
     """Algorithmic (unique-touch) bytes of one launch: each stored input
-    element read once, each output written once, at its stored type.  On a
+    element read once, each output written once, at its stored type; None for
+    kernels without a model (the team solvers, bound by latency, and the
+    V-cycles and line sweeps, modelled above).  On a
     structured box the FP64 momentum and temperature rows and the FP32
     copies are stored by direction and the solver kernels read no column
     data (the assembly reads a 4-byte direction code per row).  The pressure
@@ -166,17 +206,6 @@ def kernel_bytes(name, N, F, nnz_off):
         "bicg3_32_2_spmv": 76 * N,     # FP32: matrix 28 + 3 x 16
         "bicg3_32_3_update": 84 * N,
         "gnn_layers": 129 * N,         # one tcgen05 layer launch: h in 64, h out 64, mask 1 (four per pass)
-        # one V-cycle, per fine row.  FP32 (every level's matrix by direction;
-        # level 0's off-diagonal values read in FP16, 12 bytes), level 0:
-        # first two sweeps 24, sweep 28, restriction 28, prolongation + sweep
-        # 32, sweep 28, last sweep with r.z 28 = 168; level 1 (1/8 of the
-        # rows, about 241 bytes per row) 30; level 2 and below 4
-        "amg32_vcycle": 202 * N,
-        # FP64 (level 0 in the half form: 32 bytes of matrix per row, coarse
-        # levels by direction), level 0: first sweep 24, sweeps 4 x 56,
-        # restriction 53, prolongation 21, last sweep 56 = 378; level 1 66;
-        # level 2 and below 9
-        "amg_vcycle": 453 * N,
         "lsq_gradients_uvwpt": 208 * N,
         # a cell's faces: face index, other cell (col) and owner bits per
         # cell instead of each face's two cell indices
@@ -202,9 +231,9 @@ NCU_DRAM_BYTES_PER_ROW = {
 # Timed groups that are several kernel launches: the four layer launches of
 # the network are timed as one group.
 KERNELS_PER_GROUP = {"gnn_layers": 4}
-# Timed groups made of different kernels (one V-cycle: 25 kernels in FP32, 21
-# in FP64 on the benchmark box); they get per-group figures but are not the
-# line's roofline kernel, which is one kernel.
+# Timed groups made of different kernels (one V-cycle: 21 kernels on the
+# benchmark box); they get per-group figures but are not the line's roofline
+# kernel, which is one kernel.
 COMPOSITE = ("amg_vcycle", "amg32_vcycle")
 
 
@@ -419,24 +448,26 @@ def working_launches(name, st, launches):
     """Launches of a kernel in the instrumented pass that did work: the
     host-polled batches of that pass also launch iterations that find their
     solve converged and return at once.  One V-cycle and one product per
-    PCG iteration, one BiCGStab triple per iteration; assembly kernels run
-    once per pass."""
+    PCG iteration, one BiCGStab triple or line sweep per iteration of
+    theirs; assembly kernels run once per pass."""
     it = None
     if name in KERNELS_PER_GROUP:
         return launches * KERNELS_PER_GROUP[name]
     if name in ("amg32_vcycle", "amg_vcycle", "pcg_iter1_spmv", "pcg32_iter1_spmv"):
         it = st["pressure_iters_total"]
-    elif name.startswith("bicg3"):
+    elif name.startswith(("bicg3", "line_sweep3")):
         it = max(st["momentum_iters"])
-    elif name.startswith("bicg1"):
+    elif name.startswith(("bicg1", "line_sweep1")):
         it = st["temperature_iters"]
     if it is None or it <= 0 or it > launches:
         return launches
     return it
 
 
-def roofline_of(solver, mesh, N):
-    """One instrumented pass: for every kernel with a byte model, its
+def roofline_of(solver, mesh, N, dims, natural, sms):
+    """One instrumented pass (an event pair around every launch, so the solves are
+    host-driven batches of the same kernels and not the timed passes' device-side
+    loops and corrector graph): for every kernel with a byte model, its
     CUDA-event time, launches (all, and those that did work) and achieved
     bandwidth; the single kernel with the largest time is the line's
     roofline (a V-cycle, a group of different kernels, is listed but not
@@ -452,10 +483,17 @@ def roofline_of(solver, mesh, N):
     peak, kind = measured_peaks()
     per_kernel = {}
     for name, (ms, cnt) in kt.items():
-        b = kernel_bytes(name, N, mesh.n_faces, nnz_off)
-        if cnt == 0 or b is None:
+        if cnt == 0:
             continue
         work = working_launches(name, st, cnt)
+        if name in COMPOSITE:
+            b = vcycle_bytes(dims, name == "amg32_vcycle", sms, natural)
+        elif name.startswith("line_sweep"):
+            b = sweep_bytes(3 if name.startswith("line_sweep3") else 1, N, work)
+        else:
+            b = kernel_bytes(name, N, mesh.n_faces, nnz_off)
+        if b is None:
+            continue
         avg_s = ms / work / 1e3
         launches = cnt * KERNELS_PER_GROUP.get(name, 1)
         per_kernel[name] = {"ms": round(ms, 4), "launches": launches, "working_launches": work,
@@ -555,7 +593,9 @@ def main():
             r["e2e"] = replicas.whole_job_rate(args.steps, max_over_ranks(e0.elapsed_time(e1) / 1e3), world)
             r["e2e_bytes"] = 5 * (N + 6) * 8
         if rank == 0 and not args.no_roofline:
-            r["roofline"], r["kernel_ms"], r["kernels"] = roofline_of(solver, mesh, N)
+            r["roofline"], r["kernel_ms"], r["kernels"] = roofline_of(
+                solver, mesh, N, dims, args.reorder == "none",
+                torch.cuda.get_device_properties(local).multi_processor_count)
         runs[cfg] = r
         solver.close()
 
@@ -621,7 +661,7 @@ def main():
                                        + ("source blobs, " if args.source_period <= 0 else
                                           f"source blobs with amplitudes sin(2 pi pass / {args.source_period} + "
                                           "random phase) updated on the device every pass, ")
-                                       + f"{desc}, BiCGStab momentum/T, rtol 1e-8"
+                                       + f"{desc}, momentum/T by FP64 line sweeps, rtol 1e-8"
                                        + (", RCM cell order" if args.reorder == "rcm" else ""),
                            "cells": N, "faces": mesh.n_faces, "l2": "inputs larger than L2 (~4.5 GB working set)",
                            "parallelism": "replicas" if world > 1 else "single GPU"},
