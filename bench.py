@@ -225,6 +225,8 @@ def kernel_bytes(name, N, F, nnz_off):
 # rows to the bench size for the roofline's `traffic`.
 NCU_DRAM_BYTES_PER_ROW = {
     "bicg3_1_spmv": 217.2,   # k_bicg_1<double,3>: 384.3 MB read + written on 1,769,472 cells
+    "line_sweep3_64": 103.0,  # k_line_sweep64<3>: 83.1 MB the first sweep, 215.3 the others, four in all
+    "mass_flux": 539.1,      # k_mass_flux: 953.9 MB
     "gnn_layers": 103.6,     # k_gnn_layer_umma: 115.1 + 68.2 MB read + written on 1,769,472 cells
 }
 

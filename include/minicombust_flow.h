@@ -101,9 +101,10 @@ typedef struct mc_flow_params {
     double urf_pressure;
     double urf_temperature;
     double flux_corr;         /* non-orthogonal flux-correction factor */
-    double u_rtol;            /* momentum and temperature BiCGStab: ||r|| <= u_rtol ||b|| */
+    double u_rtol;            /* momentum, temperature and scalar solves: ||r|| <= u_rtol ||b|| */
     double p_rtol;            /* pressure-correction PCG: ||r|| <= p_rtol ||b|| */
-    int max_iters;            /* per Krylov solve */
+    int max_iters;            /* per Krylov solve; also bounds the x-line sweeps of MC_PRECISION_FP64, which are
+                                 used from 50 up */
     int pressure_solver;      /* MC_PSOLVER_* */
     int precision;            /* MC_PRECISION_* */
     int initial_guess;        /* MC_GUESS_* for the first pressure correction of a pass (later ones start at 0) */
@@ -128,7 +129,7 @@ typedef struct mc_flow_params {
                                  two variances -- in the reference's order TE, ED, TEM, FUL, PRO,
                                  VARF, VARP (FlowSolver.inl:3229-3261).  Default: 1 in
                                  MC_MODE_COMPAT, 0 in MC_MODE_SIMPLE. */
-    int ir_line_steps;        /* MC_PRECISION_FP32_REFINED, momentum and temperature: k > 0 solves them by x-line
+    int ir_line_steps;        /* MC_PRECISION_FP32_REFINED, momentum and temperature: any k > 0 solves them by x-line
                                  sweeps in FP64 (the splitting that keeps the diagonal and the upwind -x
                                  couplings, solved along each line) on meshes whose cells run x-fastest
                                  along whole lines, as MC_PRECISION_FP64 does; 0, or another mesh: inner
@@ -137,8 +138,10 @@ typedef struct mc_flow_params {
 
 /* Per-pass statistics. */
 typedef struct mc_iter_stats {
-    int momentum_iters[3];
-    int temperature_iters;
+    int momentum_iters[3];           /* sweeps where x-line sweeps made the solve (meshes whose cells
+                                        form whole lines along x), else BiCGStab iterations (with
+                                        FP32 refinement those of the inner solves) */
+    int temperature_iters;           /* likewise */
     int pressure_solves;
     int pressure_iters_total;
     int pressure_iters_first;
@@ -152,8 +155,8 @@ typedef struct mc_iter_stats {
                                         (MC_GUESS_LEARNED) the network's prediction */
     double guess_rel_residual_first; /* ||b - A x0|| / ||b|| of that guess (1 for zero) */
     double pressure_rel_residual_first; /* ||r|| / ||b|| at the end of the first pressure solve */
-    int scalar_iters[6];             /* transport_scalars: BiCGStab iterations of TE, ED, FUL, PRO,
-                                        VARF, VARP (0 when not run) */
+    int scalar_iters[6];             /* transport_scalars: sweeps or iterations, likewise, of TE, ED,
+                                        FUL, PRO, VARF, VARP (0 when not run) */
 } mc_iter_stats;
 
 typedef struct mc_flow mc_flow;

@@ -766,7 +766,7 @@ bool amg_paired_sweeps(const AmgHierarchy &H, bool fp32) { return fp32 && H.swee
 template <typename T>
 static long tile_resident()
 {
-    return (long)krylov_grid(INT32_MAX - 256) / 8 * (sizeof(T) == 4 ? 2 : 1);
+    return (long)krylov_sms() * (sizeof(T) == 4 ? 2 : 1);
 }
 
 // Split of a box level into tile columns and planes: the one whose waves of

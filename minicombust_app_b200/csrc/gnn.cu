@@ -1378,7 +1378,7 @@ void gnn_init_params(float *p, uint64_t seed)
 void gnn_pack(cudaStream_t s, const float *p, bf16 *pk) { k_gnn_pack<<<32, 256, 0, s>>>(p, pk); }
 
 // train: keep every layer's input and relu(W1 u + c1) for the backward pass
-// (needs a work area carved with train = true); inference ping-pongs h[0],
+// (needs a work area carved for that many samples); inference ping-pongs h[0],
 // h[1] and uses the offset-form weights where the graph allows.
 template <typename T>
 static void forward_impl(cudaStream_t s, const GnnGraph &g, const GnnBatch<T> &in, int samples, const float *p,

@@ -32,7 +32,7 @@ __device__ __forceinline__ bool finite(double x) { return isfinite(x); }
 
 } // namespace
 
-static int krylov_sms()
+int krylov_sms()
 {
     static int sms = 0;
     if (sms == 0) {
@@ -1236,7 +1236,7 @@ void bir_residual(cudaStream_t s, const Ell &A, const BirVectors<R> &v)
 //
 // HBM bound: a sweep streams the row once for all R systems, 56 bytes of
 // matrix and per system b, x_k and x_{k+1} (24 bytes; 16 for the first sweep,
-// which reads three of the seven matrix values).  A momentum solve to 1e-8
+// which reads two of the seven matrix values).  A momentum solve to 1e-8
 // takes four sweeps, 448 bytes per row, where BiCGStab takes 8 to 10
 // iterations of 520: a plain FP64 timestep of the 2 x 128^3 box 48.6 -> 26.8 ms,
 // with errors against 64-bit solves ten times smaller.

@@ -301,7 +301,7 @@ struct SweepState {
 };
 // Sweep number k (0: from zero, which also sets the tolerance rtol ||b||):
 // reads x[k & 1], writes x[(k & 1) ^ 1]; sweeps after the solve is done do
-// nothing.  grid blocks of the launch: line_sweep64_grid.
+// nothing.  Blocks of the launch: at most line_sweep64_blocks.
 template <int R>
 struct SweepVectors {
     double *x[2][R];            // the two iterates
@@ -316,7 +316,8 @@ int line_sweep64_blocks(int N);  // upper bound on the blocks of a launch over N
 
 enum { KRYLOV_OK = 0, KRYLOV_NOT_CONVERGED = 1, KRYLOV_NONFINITE = 2, KRYLOV_TIMEOUT = 3 };
 
-// Grid size used by the Krylov kernels for N rows.
+// SMs of the device, and the grid size used by the Krylov kernels for N rows.
+int krylov_sms();
 int krylov_grid(int N);
 
 // Programmatic dependent launch: a kernel started with pdl_launch may be
