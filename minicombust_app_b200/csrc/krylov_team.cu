@@ -421,15 +421,19 @@ __global__ void __launch_bounds__((team_threads<CLUSTER, RPT>), 1)
 struct TeamShape {
     bool cluster = false;
     int blocks = 0, threads = 0, rows = 0, rpt = 0;
+    int smem_max = 0;  // dynamic shared memory a block may have
 };
+constexpr int TEAM_STATIC_SMEM = 2048;  // at least the static part of a team kernel
 
 TeamShape team_shape(int N)
 {
     TeamShape s;
-    int dev = 0, sms = 0;
+    int dev = 0, sms = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
         return s;
+    s.smem_max = optin - TEAM_STATIC_SMEM;
     if (N <= TEAM_CLUSTER * 1024) {
         s.cluster = true;
         s.blocks = std::max(1, N / 128);
@@ -451,7 +455,10 @@ template <typename... KArgs, typename... Args>
 bool team_launch(void (*k)(KArgs...), const TeamShape &sh, size_t smem, cudaStream_t s, unsigned int *words,
                  Args &&...args)
 {
-    bool ok = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+    // (a kernel's limit is shared by the process: always the same value, so that
+    // a thread with a smaller system does not lower another's between its two calls)
+    bool ok = smem <= (size_t)sh.smem_max &&
+              cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sh.smem_max) == cudaSuccess;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(sh.blocks);
     cfg.blockDim = dim3(sh.threads);

@@ -90,6 +90,39 @@ def test_kernel_counts_name_the_solver_that_ran(gpu, dims, team):
     s.close()
 
 
+def test_handles_of_two_sizes_in_two_threads(gpu):
+    """Two systems that run the same team kernel with different amounts of shared
+    memory: each pass is made by the team, with the bits of a pass made alone."""
+    import threading
+    boxes = ((50, 30, 30), (90, 50, 48))
+
+    def passes(dims, out):
+        s = flow.FlowSolver(flow.Mesh.box(*dims, 0.2, 0.1, 0.1), params=flow.default_params(flow.MODE_SIMPLE))
+        for name, vals in noisy_fields(s.N, 5).items():
+            a = s.field(name)
+            a[:s.N] = vals
+            s.set_field(name, a)
+        s.set_timing(True)
+        for _ in range(12):
+            s.simple_iteration()
+        n = {k: c for k, (_, c) in s.kernel_times().items()}
+        out[dims] = {f: s.field(f) for f in ("U", "P", "TEM")}, n["pcg_team"], n["pcg_iter1_spmv"]
+        s.close()
+
+    alone, together = {}, {}
+    for dims in boxes:
+        passes(dims, alone)
+    threads = [threading.Thread(target=passes, args=(dims, together)) for dims in boxes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for dims in boxes:
+        assert together[dims][1] == alone[dims][1] > 0 and together[dims][2] == alone[dims][2] == 0
+        for f, a in alone[dims][0].items():
+            assert np.array_equal(together[dims][0][f], a), (dims, f)
+
+
 CHILD = r"""
 import ctypes, os, sys
 sys.path.insert(0, os.environ["MC_ROOT"])
