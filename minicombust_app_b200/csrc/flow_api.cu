@@ -939,7 +939,7 @@ int solve_sweeps(mc_flow *h, const double *diag, const double *off, const double
     const int across = L.ex + 2 * (int)std::sqrt((double)(h->N / L.ex));  // cells of a box's three edges, about
     double before[R];                                                     // residual norms squared, a batch earlier
     for (int k = 0; k < limit;) {
-        for (int q = 0; q < SWEEP_BATCH; q++, k++)
+        for (int q = 0; q < SWEEP_BATCH && k < limit; q++, k++)
             launch(h, R == 3 ? K_SWEEP3 : K_SWEEP1, [&] { line_sweep64<R>(h->stream, L, v, k, h->prm.u_rtol); });
         const int rc = check_launch(h);
         if (rc) return rc;

@@ -94,6 +94,22 @@ def test_refined_sweeps_whatever_max_iters(gpu):
     assert 1 <= max(st.momentum_iters) <= 12 and 1 <= st.temperature_iters <= 12
 
 
+def test_sweeps_within_max_iters(gpu):
+    """A temperature solve that needs some 200 sweeps or iterations, bounded at 100."""
+    s = flow.FlowSolver(flow.Mesh.box(24, 32, 16, 0.2, 0.1, 0.1),
+                        params=flow.default_params(flow.MODE_SIMPLE, delta=1e-2, max_iters=100,
+                                                   pressure_solver=flow.PSOLVER_PCG_AMG))
+    for name, vals in noisy_initial_fields(s.N, {**BASE, "U": 1.0, "V": 80.0}, 1).items():
+        a = s.field(name)
+        a[:s.N] = vals
+        s.set_field(name, a)
+    s.set_timing(True)
+    assert s.simple_iteration(check=False) == flow.MC_ERR_NOT_CONVERGED
+    assert 0 < s.kernel_times()["line_sweep1_64"][1] <= 100 and s.last_stats.temperature_iters <= 100
+    assert max(s.last_stats.momentum_iters) <= 100
+    s.close()
+
+
 def test_long_step_cross_flow_matches_oracle(gpu):
     run_both((12, 24, 6), passes=1, base={**BASE, "U": 1.0, "V": 80.0}, delta=1e-2)
 
